@@ -218,7 +218,7 @@ __device__ __forceinline__ void ausm_plus_flux(float rhoL, float unL, float utL,
 }
 
 // One face of computeFluxesKernel (x: src/solver.cu:1502-1598, y: :1601-1682)
-// from the two cells a | b and their half limited slopes sa, sb:
+// from the two cells a | b and their limited slopes sa, sb (cell_slopes):
 // MUSCL reconstruction of (rho, u, v, p), clamps, Riemann flux and the
 // upwinded rho_e flux.  `valid`: neither a nor b is a wall; `near_wall`:
 // first order (a wall at the outer stencil cells; the density test is done
@@ -231,14 +231,14 @@ __device__ __forceinline__ void face_flux_sl(bool valid, bool near_wall, const P
         float order_mask = (near_wall || lowDensity) ? 0.0f : 1.0f;
         const float aa = XDIR ? a.u : a.v, ab = XDIR ? b.u : b.v;
         const float ta = XDIR ? a.v : a.u, tb = XDIR ? b.v : b.u;
-        float rhoL = a.rho + sa[0] * order_mask;
-        float unL = aa + sa[1] * order_mask;
-        float utL = ta + sa[2] * order_mask;
-        float pL = a.p + sa[3] * order_mask;
-        float rhoR = b.rho - sb[0] * order_mask;
-        float unR = ab - sb[1] * order_mask;
-        float utR = tb - sb[2] * order_mask;
-        float pR = b.p - sb[3] * order_mask;
+        float rhoL = a.rho + 0.5f * sa[0] * order_mask;
+        float unL = aa + 0.5f * sa[1] * order_mask;
+        float utL = ta + 0.5f * sa[2] * order_mask;
+        float pL = a.p + 0.5f * sa[3] * order_mask;
+        float rhoR = b.rho - 0.5f * sb[0] * order_mask;
+        float unR = ab - 0.5f * sb[1] * order_mask;
+        float utR = tb - 0.5f * sb[2] * order_mask;
+        float pR = b.p - 0.5f * sb[3] * order_mask;
         rhoL = fmaxf(rhoL, MIN_DENSITY);
         pL = fmaxf(pL, MIN_PRESSURE);
         rhoR = fmaxf(rhoR, MIN_DENSITY);

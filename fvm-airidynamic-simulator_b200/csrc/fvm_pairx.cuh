@@ -48,19 +48,17 @@ __device__ __forceinline__ f2 p_div(f2 a, f2 b) { return p_mul(a, p_rcp(b)); }
 __device__ __forceinline__ f2 p_rsqrt(f2 a) { return mk2(rsqrtf(a.x), rsqrtf(a.y)); }
 __device__ __forceinline__ f2 p_sel(bool cx, bool cy, f2 a, f2 b) { return mk2(cx ? a.x : b.x, cy ? a.y : b.y); }
 
-// Half the limited slope per lane, (q_i+1/2 - q_i) of the reconstruction:
-// minmod (src/solver.cu:110-150) or the van Leer harmonic mean.  The limiters'
-// own factors absorb the half: 0.25 (sign + sign) min, and ab / (a + b).
+// Limited slope per lane (as limited_slope).
 template <int LIM>
-__device__ __forceinline__ f2 p_half_slope(f2 qm1, f2 q0, f2 qp1) {
+__device__ __forceinline__ f2 p_slope(f2 qm1, f2 q0, f2 qp1) {
     const f2 dL = p_sub(q0, qm1), dR = p_sub(qp1, q0);
     if (LIM == 0) {
-        const f2 s = p_add(mk2(copysignf(0.25f, dL.x), copysignf(0.25f, dL.y)),
-                           mk2(copysignf(0.25f, dR.x), copysignf(0.25f, dR.y)));
+        const f2 s = p_mul(splat(0.5f), p_add(mk2(copysignf(1.0f, dL.x), copysignf(1.0f, dL.y)),
+                                               mk2(copysignf(1.0f, dR.x), copysignf(1.0f, dR.y))));
         return p_mul(s, mk2(fminf(fabsf(dL.x), fabsf(dR.x)), fminf(fabsf(dL.y), fabsf(dR.y))));
     } else {
         const f2 ab = p_mul(dL, dR);
-        const f2 q = p_div(ab, p_add(dL, dR));
+        const f2 q = p_div(p_mul(splat(2.0f), ab), p_add(dL, dR));
         return mk2(ab.x > 0.0f ? q.x : 0.0f, ab.y > 0.0f ? q.y : 0.0f);
     }
 }
@@ -73,108 +71,109 @@ __device__ __forceinline__ PairPrim pair_prim(const float4 &A, const float4 &B) 
     return PairPrim{mk2(A.x, A.y), mk2(A.z, A.w), mk2(B.x, B.y), mk2(B.z, B.w)};
 }
 
-// Half limited slopes of a cell pair in the face frame: normal and tangential
+// Limited slopes of a cell pair in the face frame: normal and tangential
 // velocity components (x-faces: u, v; y-faces: v, u).
 struct PairSl {
     f2 rho, n, t, p;
 };
 
 // Two faces between cells a | b (lane .x: face 0, lane .y: face 1) from the
-// cells' primitives and half limited slopes sa, sb (face frame); F = {mass,
+// cells' primitives and limited slopes sa, sb (face frame); F = {mass,
 // x-momentum, y-momentum, energy, rho_e}, each a lane pair.  valid*: neither
 // side a wall; near*: first order (wall at the outer stencil cells).
-//
-// The stage kernels are bound by issue slots, so the HLLC flux is written in
-// the form with the fewest operations (157 issued per face pair, counted in
-// the source; the operation-for-operation form of the reference takes 195):
-//  * Roe sound speed from c~^2 = wL cL^2 + wR cR^2 + (gamma-1)/2 wL wR |dV|^2
-//    with wK = sqrt(rho_K) / (sqrt(rho_L) + sqrt(rho_R)), the identity that
-//    H~ - |V~|^2/2 expands to: no enthalpies, no cancellation, positive, so the
-//    reference's fallback for c~^2 <= 0 has no case left;
-//  * S* - u_L = (dp - m_R dn) / (m_L - m_R), m_K = rho_K (S_K - u_K);
-//  * across the wave S_K the star flux F_K + S_K (U* - U_K) of the reference
-//    equals {F0, F0 S* + p*, F0 u_t, (E* + p*) S*} with F0 = r S* + S_K
-//    (rho* - r), r the star density before its floor, p* of the momentum
-//    before its floor and p* of the energy after it: the same values with
-//    the floors acting, and no difference of large terms where S* is small;
-//  * a supersonic face takes S* = u_K in the same expressions, which then
-//    give F_K.
-// Measured at 8192x4096, van Leer (SM clock 1965 MHz): stage 1 / stage 2
-// 695 / 696 us with the reference's form, 644 / 658 us with this one.
 template <bool XDIR>
 __device__ __forceinline__ void face_pair_core(bool valid0, bool near0, bool valid1, bool near1, const PairPrim &a,
                                                const PairSl &sa, const PairPrim &b, const PairSl &sb, f2 F[5]) {
     const bool fo0 = near0 || a.rho.x < LOW_DENSITY || b.rho.x < LOW_DENSITY;
     const bool fo1 = near1 || a.rho.y < LOW_DENSITY || b.rho.y < LOW_DENSITY;
-    const f2 om = mk2(fo0 ? 0.0f : 1.0f, fo1 ? 0.0f : 1.0f);  // order mask
-    const f2 omn = mk2(fo0 ? 0.0f : -1.0f, fo1 ? 0.0f : -1.0f);
+    const f2 hp = splat(0.5f);
+    const f2 omh = mk2(fo0 ? 0.0f : 0.5f, fo1 ? 0.0f : 0.5f);  // half order mask
     const f2 an = XDIR ? a.u : a.v, at = XDIR ? a.v : a.u;
     const f2 bn = XDIR ? b.u : b.v, bt = XDIR ? b.v : b.u;
     // MUSCL: left = a + slope_a/2, right = b - slope_b/2
-    const f2 rL = p_max(p_fma(sa.rho, om, a.rho), MIN_DENSITY);
-    const f2 nL = p_fma(sa.n, om, an);
-    const f2 tL = p_fma(sa.t, om, at);
-    const f2 pL = p_max(p_fma(sa.p, om, a.p), MIN_PRESSURE);
-    const f2 rR = p_max(p_fma(sb.rho, omn, b.rho), MIN_DENSITY);
-    const f2 nR = p_fma(sb.n, omn, bn);
-    const f2 tR = p_fma(sb.t, omn, bt);
-    const f2 pR = p_max(p_fma(sb.p, omn, b.p), MIN_PRESSURE);
+    f2 rL = p_fma(sa.rho, omh, a.rho);
+    const f2 nL = p_fma(sa.n, omh, an);
+    const f2 tL = p_fma(sa.t, omh, at);
+    f2 pL = p_fma(sa.p, omh, a.p);
+    const f2 omm = mk2(-omh.x, -omh.y);
+    f2 rR = p_fma(sb.rho, omm, b.rho);
+    const f2 nR = p_fma(sb.n, omm, bn);
+    const f2 tR = p_fma(sb.t, omm, bt);
+    f2 pR = p_fma(sb.p, omm, b.p);
+    rL = p_max(rL, MIN_DENSITY);
+    pL = p_max(pL, MIN_PRESSURE);
+    rR = p_max(rR, MIN_DENSITY);
+    pR = p_max(pR, MIN_PRESSURE);
+    // E = p/(gamma-1) + rho*(u^2 + v^2)/2, the x component squared first
+    const f2 igm1 = splat(1.0f / (GAMMA - 1.0f));
+    const f2 eL = p_mul(pL, igm1), eR = p_mul(pR, igm1);
+    const f2 qL = XDIR ? p_fma(nL, nL, p_mul(tL, tL)) : p_fma(tL, tL, p_mul(nL, nL));
+    const f2 qR = XDIR ? p_fma(nR, nR, p_mul(tR, tR)) : p_fma(tR, tR, p_mul(nR, nR));
+    const f2 EL = p_fma(p_mul(hp, rL), qL, eL);
+    const f2 ER = p_fma(p_mul(hp, rR), qR, eR);
 
-    // ---- wave speeds: Roe-averaged Davis bounds with the entropy fix.  One
-    // reciprocal square root per side gives sqrt(rho) = rho / sqrt(rho) and
-    // 1/rho = (1/sqrt(rho))^2; the densities are >= MIN_DENSITY, so the
-    // reference's 1e-10 in the weights' divisor is below its last bit
+    // ---- HLLC with Roe-averaged Davis wave speeds; quotients that share a
+    // divisor (1/rho of each side, the Roe weight sum, the star-state
+    // denominator) multiply by one reciprocal
+    // one reciprocal square root per side gives sqrt(rho) = rho / sqrt(rho)
+    // and 1/rho = (1/sqrt(rho))^2
     const f2 rqL = p_rsqrt(rL), rqR = p_rsqrt(rR);
     const f2 sqL = p_mul(rL, rqL), sqR = p_mul(rR, rqR);
-    const f2 cL2 = p_mul(p_mul(splat(GAMMA), pL), p_mul(rqL, rqL));
-    const f2 cR2 = p_mul(p_mul(splat(GAMMA), pR), p_mul(rqR, rqR));
-    const f2 cL = p_sqrt(cL2), cR = p_sqrt(cR2);
-    const f2 wR = p_mul(sqR, p_rcp(p_add(sqL, sqR)));
-    const f2 wL = p_fma(wR, splat(-1.0f), splat(1.0f));
-    const f2 dn = p_sub(nR, nL), dt = p_sub(tR, tL);
-    const f2 un_roe = p_fma(wR, dn, nL);
-    const f2 d2 = p_fma(dn, dn, p_mul(dt, dt));
-    const f2 ww = p_mul(wL, p_mul(splat(0.5f * (GAMMA - 1.0f)), wR));
-    const f2 c_roe = p_sqrt(p_fma(ww, d2, p_fma(wR, cR2, p_mul(wL, cL2))));
+    const f2 irL = p_mul(rqL, rqL), irR = p_mul(rqR, rqR);
+    const f2 cL = p_sqrt(p_mul(p_mul(splat(GAMMA), pL), irL));
+    const f2 cR = p_sqrt(p_mul(p_mul(splat(GAMMA), pR), irR));
+    const f2 iden = p_rcp(p_add(p_add(sqL, sqR), splat(1e-10f)));
+    const f2 un_roe = p_mul(p_fma(sqL, nL, p_mul(sqR, nR)), iden);
+    const f2 ut_roe = p_mul(p_fma(sqL, tL, p_mul(sqR, tR)), iden);
+    const f2 HL = p_mul(p_add(EL, pL), irL), HR = p_mul(p_add(ER, pR), irR);
+    const f2 H_roe = p_mul(p_fma(sqL, HL, p_mul(sqR, HR)), iden);
+    const f2 q_roe = XDIR ? p_fma(un_roe, un_roe, p_mul(ut_roe, ut_roe)) : p_fma(ut_roe, ut_roe, p_mul(un_roe, un_roe));
+    const f2 c2 = p_mul(splat(GAMMA - 1.0f), p_fma(splat(-0.5f), q_roe, H_roe));
+    const f2 c_avg = p_mul(hp, p_add(cL, cR));
+    const f2 c_roe = mk2(c2.x > 0.0f ? sqrtf(c2.x) : c_avg.x, c2.y > 0.0f ? sqrtf(c2.y) : c_avg.y);
     f2 SL = p_min(p_sub(nL, cL), p_sub(un_roe, c_roe));
     f2 SR = p_max(p_add(nR, cR), p_add(un_roe, c_roe));
     const f2 delta = p_mul(splat(ENTROPY_FIX), p_max(cL, cR));
     SL = mk2(fabsf(SL.x) < delta.x ? -delta.x : SL.x, fabsf(SL.y) < delta.y ? -delta.y : SL.y);
     SR = mk2(fabsf(SR.x) < delta.x ? delta.x : SR.x, fabsf(SR.y) < delta.y ? delta.y : SR.y);
-    // contact speed: m_L - m_R < 0 always (S_L <= u_L - c_L, S_R >= u_R + c_R),
-    // so the reference's floor of its magnitude is a minimum
-    const f2 mL = p_mul(rL, p_sub(SL, nL)), nmR = p_mul(rR, p_sub(nR, SR));
-    f2 ds = p_add(mL, nmR);
-    ds = mk2(fminf(ds.x, -1e-10f), fminf(ds.y, -1e-10f));
-    const f2 Ss = p_fma(p_fma(nmR, dn, p_sub(pR, pL)), p_rcp(ds), nL);
-    // upwind side K of the wave fan: L if all waves move right (S_L >= 0) or
-    // the contact does (S* >= 0), R otherwise; one evaluation on K's operands
-    // gives the value of the reference's four-way branch (src/solver.cu:1160-1222)
+    const f2 aL = p_sub(SL, nL), aR = p_sub(SR, nR);
+    const f2 mL = p_mul(rL, aL), mR = p_mul(rR, aR);
+    const f2 ds = p_sub(mL, mR);
+    const f2 sds = mk2(copysignf(fmaxf(fabsf(ds.x), 1e-10f), ds.x), copysignf(fmaxf(fabsf(ds.y), 1e-10f), ds.y));
+    const f2 Ss = p_div(p_sub(p_fma(mL, nL, p_sub(pR, pL)), p_mul(mR, nR)), sds);
+    // upwind side K of the wave fan (see hllc_flux)
     const bool supL0 = SL.x >= 0.0f, supL1 = SL.y >= 0.0f;
     const bool supR0 = !supL0 && SR.x <= 0.0f, supR1 = !supL1 && SR.y <= 0.0f;
     const bool useL0 = supL0 || (!supR0 && Ss.x >= 0.0f), useL1 = supL1 || (!supR1 && Ss.y >= 0.0f);
     const f2 rK = p_sel(useL0, useL1, rL, rR), nK = p_sel(useL0, useL1, nL, nR), tK = p_sel(useL0, useL1, tL, tR);
-    const f2 pK = p_sel(useL0, useL1, pL, pR), SK = p_sel(useL0, useL1, SL, SR);
-    const f2 Sx = p_sel(supL0 || supR0, supL1 || supR1, nK, Ss);
-    const f2 igm1 = splat(1.0f / (GAMMA - 1.0f));
-    const f2 EK = p_fma(p_mul(splat(0.5f), rK), p_fma(nK, nK, p_mul(tK, tK)), p_mul(pK, igm1));
-    // mass flux through the wave S_K; |S* - S_K| floored at 1e-10 with its sign
-    const f2 e = p_sub(nK, SK);
-    const f2 g = p_mul(rK, e);
-    f2 cd = p_sub(Sx, SK);
+    const f2 pK = p_sel(useL0, useL1, pL, pR), EK = p_sel(useL0, useL1, EL, ER), SK = p_sel(useL0, useL1, SL, SR);
+    const f2 d = p_sub(SK, nK);   // SK - unK
+    const f2 rkd = p_mul(rK, d);  // rK (SK - unK): the same product as mL / mR
+    const f2 fK0 = p_mul(rK, nK);
+    const f2 fK1 = p_fma(fK0, nK, pK);
+    const f2 fK2 = XDIR ? p_mul(fK0, tK) : p_mul(p_mul(rK, tK), nK);  // (rho u) v either way
+    const f2 fK3 = p_mul(p_add(EK, pK), nK);
+    // |S_K - S*| floored at 1e-10 with its sign (the reference's
+    // `cd >= 0 ? 1e-10 : -1e-10`; S_K is never zero after the entropy fix,
+    // so the difference is never -0)
+    f2 cd = p_sub(SK, Ss);
     cd = mk2(copysignf(fmaxf(fabsf(cd.x), 1e-10f), cd.x), copysignf(fmaxf(fabsf(cd.y), 1e-10f), cd.y));
     const f2 icd = p_rcp(cd);
-    const f2 r0 = p_mul(g, icd);
-    const f2 F0 = p_fma(SK, p_sub(p_max(r0, MIN_DENSITY), r0), p_mul(r0, Sx));
-    const f2 p0 = p_fma(g, p_sub(nK, Sx), pK);
-    const f2 ps = p_max(p0, MIN_PRESSURE);
-    const f2 Fn = p_fma(F0, Sx, p0);
-    const f2 Ft = p_mul(F0, tK);
-    const f2 Es = p_mul(p_sub(p_fma(EK, e, p_mul(pK, nK)), p_mul(ps, Sx)), icd);
-    const f2 F3 = p_mul(p_add(Es, ps), Sx);
-    // upwinded internal-energy flux, by the sign of 0.5 (u_L + u_R)
-    const f2 uf = p_add(nL, nR);
-    const f2 F4 = p_mul(igm1, p_sel(uf.x >= 0.0f, uf.y >= 0.0f, p_mul(pL, nL), p_mul(pR, nR)));
+    const f2 rs = p_max(p_mul(rkd, icd), MIN_DENSITY);
+    const f2 ps = p_max(p_fma(rkd, p_sub(Ss, nK), pK), MIN_PRESSURE);
+    const f2 Es = p_mul(p_sub(p_fma(EK, d, p_mul(ps, Ss)), p_mul(pK, nK)), icd);
+    // star region: F = F_K + S_K (U*_K - U_K); supersonic: F = F_K, written
+    // as F_K + 0 * (U*_K - U_K) (there the wave fan keeps |ds| >= rho c, so
+    // the star quantities are finite and the product is exactly zero)
+    const bool st0 = !(supL0 || supR0), st1 = !(supL1 || supR1);
+    const f2 SKs = p_sel(st0, st1, SK, splat(0.0f));
+    const f2 F0 = p_fma(SKs, p_sub(rs, rK), fK0);
+    const f2 Fn = p_fma(SKs, p_sub(p_mul(rs, Ss), fK0), fK1);
+    const f2 Ft = p_fma(SKs, p_mul(p_sub(rs, rK), tK), fK2);
+    const f2 F3 = p_fma(SKs, p_sub(Es, EK), fK3);
+    // upwinded internal-energy flux
+    const f2 uf = p_add(nL, nR);  // sign of 0.5 (unL + unR)
+    const f2 F4 = p_sel(uf.x >= 0.0f, uf.y >= 0.0f, p_mul(eL, nL), p_mul(eR, nR));
     const f2 Fx = XDIR ? Fn : Ft, Fy = XDIR ? Ft : Fn;
     // wall faces: no mass/energy flux, normal momentum flux = pressure of the left/bottom cell
     const f2 zero = splat(0.0f);
@@ -191,14 +190,14 @@ __device__ __forceinline__ void pair_from_lanes(const float f0[5], const float f
     for (int k = 0; k < 5; k++) F[k] = mk2(f0[k], f1[k]);
 }
 
-// Half limited x-slopes of a row pair from the slope ring's interleaved entries
+// Limited x-slopes of a row pair from the slope ring's interleaved entries
 // {rho_r, rho_r+1, u_r, u_r+1}, {v_r, v_r+1, p_r, p_r+1} (x-face frame).
 __device__ __forceinline__ PairSl pair_sl(const float4 &A, const float4 &B) {
     return PairSl{mk2(A.x, A.y), mk2(A.z, A.w), mk2(B.x, B.y), mk2(B.z, B.w)};
 }
 
 // x-faces of rows r (lane .x) and r+1 (lane .y) between cells a | b from
-// their primitives and half limited x-slopes sa, sb.
+// their primitives and limited x-slopes sa, sb.
 template <int SCHEME>
 __device__ __forceinline__ void face_pair_x_sl(bool valid0, bool near0, bool valid1, bool near1, const PairPrim &a,
                                                const PairSl &sa, const PairPrim &b, const PairSl &sb, f2 F[5]) {
@@ -224,9 +223,9 @@ __device__ __forceinline__ void face_pair_x_sl(bool valid0, bool near0, bool val
 template <int SCHEME, int LIM>
 __device__ __forceinline__ void face_pair_y(bool valid0, bool near0, bool valid1, bool near1, const PairPrim &lo,
                                             const PairPrim &mid, const PairPrim &hi, float sy_lo[4], f2 F[5]) {
-    // half slopes of rows (r-1, r): limited(row-1, row, row+1), face frame (v normal, u tangential)
-    const PairSl sm{p_half_slope<LIM>(lo.rho, mid.rho, hi.rho), p_half_slope<LIM>(lo.v, mid.v, hi.v),
-                    p_half_slope<LIM>(lo.u, mid.u, hi.u), p_half_slope<LIM>(lo.p, mid.p, hi.p)};
+    // slopes of rows (r-1, r): limited(row-1, row, row+1), face frame (v normal, u tangential)
+    const PairSl sm{p_slope<LIM>(lo.rho, mid.rho, hi.rho), p_slope<LIM>(lo.v, mid.v, hi.v),
+                    p_slope<LIM>(lo.u, mid.u, hi.u), p_slope<LIM>(lo.p, mid.p, hi.p)};
     // slopes of rows (r-2, r-1)
     const PairSl sl{mk2(sy_lo[0], sm.rho.x), mk2(sy_lo[1], sm.n.x), mk2(sy_lo[2], sm.t.x), mk2(sy_lo[3], sm.p.x)};
     if (SCHEME != 0) {  // AUSM+: per lane through the scalar path

@@ -395,8 +395,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         if (t < NT - 2) {
             const float4 *A = PA + s0 * NT + t, *B = PB + s0 * NT + t;
             const PairPrim m = pair_prim(A[0], B[0]), c = pair_prim(A[1], B[1]), p = pair_prim(A[2], B[2]);
-            const f2 sr = p_half_slope<LIM>(m.rho, c.rho, p.rho), su = p_half_slope<LIM>(m.u, c.u, p.u);
-            const f2 sv = p_half_slope<LIM>(m.v, c.v, p.v), sp = p_half_slope<LIM>(m.p, c.p, p.p);
+            const f2 sr = p_slope<LIM>(m.rho, c.rho, p.rho), su = p_slope<LIM>(m.u, c.u, p.u);
+            const f2 sv = p_slope<LIM>(m.v, c.v, p.v), sp = p_slope<LIM>(m.p, c.p, p.p);
             SA[t + 1] = make_float4(sr.x, sr.y, su.x, su.y);
             SB[t + 1] = make_float4(sv.x, sv.y, sp.x, sp.y);
         }
