@@ -74,6 +74,8 @@ constexpr int kBox = 132;
 // TMA tensor-copy destinations must be 128-byte aligned: each staged box
 // ([5][kBox] floats = 2640 B) occupies a 2688-byte (672-float) stride.
 constexpr int kBoxStride = 672;
+// class bits of both cells of a mask word (zero: two fluid cells)
+constexpr uint32_t kTypeBits = (7u << MB_TYPE_SHIFT) * 0x0101u;
 constexpr size_t align128(size_t b) { return (b + 127) & ~(size_t)127; }
 
 // Address of (field f, staged column x) in a ring slot of NB boxes.
@@ -131,7 +133,7 @@ struct StageLayout {
     // face velocity}, three float4 planes
     static constexpr size_t x_bytes = (size_t)XP * 3 * NT * 16;
     static constexpr size_t m_off = x_off + x_bytes;
-    static constexpr size_t m_bytes = (size_t)PP * 2 * NT;
+    static constexpr size_t m_bytes = (size_t)PP * 2 * NT;  // one 16-bit word per column and row pair
     static constexpr size_t bar_off = (m_off + m_bytes + 15) & ~(size_t)15;
     static constexpr int NBAR = KP + (STAGE == 2 ? 1 : 0);  // input pairs + the blend pair
     static constexpr size_t total = bar_off + NBAR * 8 + 128;  // + alignment slack
@@ -197,7 +199,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
     float4 *XA = reinterpret_cast<float4 *>(smem + L::x_off);  // [column]: mass, x-momentum
     float4 *XB = XA + NT;                                         // y-momentum, energy
     float4 *XC = XB + NT;                                         // rho_e flux, face velocity
-    uint8_t *M = smem + L::m_off;
+    // mask bytes of a row pair in one word per column: row r in bits 0-7, r+1 in 8-15
+    uint16_t *M = reinterpret_cast<uint16_t *>(smem + L::m_off);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::bar_off);
     uint64_t *bbar = bars + KP;  // blend pair (stage 2)
 
@@ -257,7 +260,7 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
     float *outp = a.out + iu;
 
     int kr = base % KP, par = (base / KP) & 1, ku = (base + KP - 1) % KP;
-    int pc0 = 0, pc1 = 2;  // P/M rows of row pairs q, q-1
+    int s0 = 0, s1 = 1;  // primitive / mask ring slots of row pairs q, q-1
     float fyB[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // y-face below row r-2
     float vfB = 0.0f;                                // and its face velocity
     float sy2[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // y-slopes of row r-2
@@ -268,7 +271,6 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         const uint32_t nA = __ldg(mcol + (size_t)clampi(r + 2, 0, ny - 1) * g.pitch);
         const uint32_t nB = __ldg(mcol + (size_t)clampi(r + 3, 0, ny - 1) * g.pitch);
         // ---- phase 1: primitives + masks of rows r, r+1
-        const int s0 = pc0 >> 1, s1 = pc1 >> 1;  // pair slots of q, q-1
         bool ok = mbar_wait_bounded(&bars[kr], (uint32_t)par);
         if (STAGE == 2 && q >= 2) ok = ok && mbar_wait_bounded(bbar, (uint32_t)((bbase + q - 2) & 1));
         if (ok) {
@@ -280,8 +282,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
                 rho[h] = ring_at<L::NB>(src, 0, rc_t);
                 prim_from_cons(rho[h], ring_at<L::NB>(src, 1, rc_t), ring_at<L::NB>(src, 2, rc_t),
                                ring_at<L::NB>(src, 3, rc_t), ring_at<L::NB>(src, 4, rc_t), u[h], v[h], p[h], T);
-                M[(pc0 + h) * NT + t] = (uint8_t)(h ? mB : mA);
             }
+            M[s0 * NT + t] = (uint16_t)(mA | (mB << 8));
             PA[s0 * NT + t] = make_float4(rho[0], rho[1], u[0], u[1]);
             PB[s0 * NT + t] = make_float4(v[0], v[1], p[0], p[1]);
         }
@@ -297,8 +299,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         // row r-2 it leaves at zero feed only the unused face (j0-2 | j0-1)).
         // Stage 1 only: in stage 2 the extra path cost more than it saved.
         if (STAGE == 1 && q == 0) {
-            pc1 = pc0;
-            pc0 = 2 - pc0;
+            s1 = s0;
+            s0 ^= 1;
             kr = ring_next<KP>(kr);
             par ^= (kr == 0) ? 1 : 0;
             ku = ring_next<KP>(ku);
@@ -310,12 +312,11 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         const float4 A0 = PA[s0 * NT + cy], B0 = PB[s0 * NT + cy];
         // y-faces (r-2 | r-1), (r-1 | r) as one lane pair; the y-slopes of row
         // r-2 are those of row r in step q-1
-        const uint32_t my0 = M[pc1 * NT + cy], my1 = M[(pc1 + 1) * NT + cy];
+        const uint32_t my = M[s1 * NT + cy];
         const PairPrim lo = pair_prim(A1, B1), hi = pair_prim(A0, B0);
         const PairPrim mid{mk2(A1.y, A0.x), mk2(A1.w, A0.z), mk2(B1.y, B0.x), mk2(B1.w, B0.z)};
         f2 Fy[5];
-        face_pair_y<SCHEME, LIM>((my0 & MB_YV) != 0, (my0 & MB_YN) != 0, (my1 & MB_YV) != 0, (my1 & MB_YN) != 0, lo,
-                                 mid, hi, sy2, Fy);
+        face_pair_y<SCHEME, LIM>(my, lo, mid, hi, sy2, Fy);
         // their face velocities (the face below row r-2 is carried)
         const f2 vfy = p_face_velocity(Fy[0], lo.rho, mid.rho);
         {
@@ -341,8 +342,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
                 const bool ey0 = (u0 == 0 || u0 == ny - 1), ey1 = (u0 + 1 == 0 || u0 + 1 == ny - 1);
                 update_pair(Uc, dX, dY, du, dv, mk2(B1.z, B1.w), edge_x, ey0, ey1, ua, Un);
                 // wall cells keep their state
-                const bool w0 = (my0 & MB_WALL) != 0, w1 = (my1 & MB_WALL) != 0;
-                if (w0 || w1) {
+                if ((my & (MB_WALL * 0x0101u)) != 0u) {
+                    const bool w0 = (my & MB_WALL) != 0u, w1 = (my & (MB_WALL << 8)) != 0u;
 #pragma unroll
                     for (int k = 0; k < 5; k++) Un[k] = p_sel(w0, w1, Uc[k], Un[k]);
                 }
@@ -352,32 +353,44 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
                     for (int k = 0; k < 5; k++)
                         Un[k] = p_fma(splat(0.5f), Un[k], p_mul(splat(0.5f), mk2(b[k * W], b[L::BSLOT + k * W])));
                 }
+// phase-1 conditions act only on non-fluid cells and the domain's edge cells
+                const uint32_t ct0 = mb_type(my), ct1 = mb_type(my >> 8);
+                if (a.apply_bc && ((my & kTypeBits) != 0u || edge_x || ey0 || ey1)) {
+                    float Ur[2][5];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    if (!(h ? st1 : st0)) continue;
-                    const int urow = u0 + h;
-                    float Ur[5];
-#pragma unroll
-                    for (int k = 0; k < 5; k++) Ur[k] = h ? Un[k].y : Un[k].x;
-                    const uint32_t ctype = mb_type(h ? my1 : my0);
-                    // phase-1 conditions act only on non-fluid cells and the domain's edge cells
-                    if (a.apply_bc && (ctype != CT_FLUID || edge_x || (h ? ey1 : ey0)))
-                        bc_pointwise(Ur, ctype, iu, urow, nx, ny, a.fs);
-                    if (a.cfl && ctype != CT_GHOST) {
-                        float uu, vv, pp, TT;
-                        prim_from_cons(Ur[0], Ur[1], Ur[2], Ur[3], Ur[4], uu, vv, pp, TT);
-                        lmax_speed = fmaxf(lmax_speed, wave_speed(uu, vv, pp, Ur[0]));
-                        nbad += nonfinite5(Ur);
+                    for (int k = 0; k < 5; k++) {
+                        Ur[0][k] = Un[k].x;
+                        Ur[1][k] = Un[k].y;
                     }
-                    float *dst = outp + (size_t)urow * g.pitch;
+                    if (st0) bc_pointwise(Ur[0], ct0, iu, u0, nx, ny, a.fs);
+                    if (st1) bc_pointwise(Ur[1], ct1, iu, u0 + 1, nx, ny, a.fs);
 #pragma unroll
-                    for (int k = 0; k < 5; k++) dst[k * g.plane] = Ur[k];
-                    // a registered display field of the step's result (the descriptor
-                    // is read here, not held in registers across the loop)
-                    if (DISP && STAGE == 2) {
-                        float *const dptr = a.disp->ptr;
-                        if (dptr)
-                            dptr[(size_t)urow * nx + iu] = derived_value(a.disp->kind, Ur[0], Ur[1], Ur[2], Ur[4]);
+                    for (int k = 0; k < 5; k++) Un[k] = mk2(Ur[0][k], Ur[1][k]);
+                }
+                if (a.cfl) {
+                    const f2 ws = pair_wave_speed(Un);
+                    const bool c0 = st0 && ct0 != CT_GHOST, c1 = st1 && ct1 != CT_GHOST;
+                    lmax_speed = fmaxf(lmax_speed, fmaxf(c0 ? ws.x : 0.0f, c1 ? ws.y : 0.0f));
+                    nbad += pair_nonfinite(Un, c0, c1);
+                }
+                float *dst = outp + (size_t)u0 * g.pitch;
+                if (st0) {
+#pragma unroll
+                    for (int k = 0; k < 5; k++) dst[k * g.plane] = Un[k].x;
+                }
+                if (st1) {
+#pragma unroll
+                    for (int k = 0; k < 5; k++) dst[k * g.plane + g.pitch] = Un[k].y;
+                }
+                // a registered display field of the step's result (the descriptor
+                // is read here, not held in registers across the loop)
+                if (DISP && STAGE == 2) {
+                    float *const dptr = a.disp->ptr;
+                    if (dptr) {
+                        const int kind = a.disp->kind;
+                        float *d = dptr + (size_t)u0 * nx + iu;
+                        if (st0) d[0] = derived_value(kind, Un[0].x, Un[1].x, Un[2].x, Un[4].x);
+                        if (st1) d[nx] = derived_value(kind, Un[0].y, Un[1].y, Un[2].y, Un[4].y);
                     }
                 }
             }
@@ -395,8 +408,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         if (t < NT - 2) {
             const float4 *A = PA + s0 * NT + t, *B = PB + s0 * NT + t;
             const PairPrim m = pair_prim(A[0], B[0]), c = pair_prim(A[1], B[1]), p = pair_prim(A[2], B[2]);
-            const f2 sr = p_slope<LIM>(m.rho, c.rho, p.rho), su = p_slope<LIM>(m.u, c.u, p.u);
-            const f2 sv = p_slope<LIM>(m.v, c.v, p.v), sp = p_slope<LIM>(m.p, c.p, p.p);
+            const f2 sr = p_half_slope<LIM>(m.rho, c.rho, p.rho), su = p_half_slope<LIM>(m.u, c.u, p.u);
+            const f2 sv = p_half_slope<LIM>(m.v, c.v, p.v), sp = p_half_slope<LIM>(m.p, c.p, p.p);
             SA[t + 1] = make_float4(sr.x, sr.y, su.x, su.y);
             SB[t + 1] = make_float4(sv.x, sv.y, sp.x, sp.y);
         }
@@ -421,10 +434,9 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
         if (xrows) {
             f2 Fx[5];
             const float4 *A = PA + s0 * NT, *B = PB + s0 * NT;
-            const uint32_t mb0 = M[pc0 * NT + tx + 1], mb1 = M[(pc0 + 1) * NT + tx + 1];
             const PairPrim ca = pair_prim(A[tx + 1], B[tx + 1]), cb = pair_prim(A[tx + 2], B[tx + 2]);
-            face_pair_x_sl<SCHEME>((mb0 & MB_XV) != 0, (mb0 & MB_XN) != 0, (mb1 & MB_XV) != 0, (mb1 & MB_XN) != 0, ca,
-                                   pair_sl(SA[tx + 1], SB[tx + 1]), cb, pair_sl(SA[tx + 2], SB[tx + 2]), Fx);
+            face_pair_core<true, SCHEME>(M[s0 * NT + tx + 1], ca, pair_sl(SA[tx + 1], SB[tx + 1]), cb,
+                                         pair_sl(SA[tx + 2], SB[tx + 2]), Fx);
             if (t <= W) {
                 XA[t] = make_float4(Fx[0].x, Fx[0].y, Fx[1].x, Fx[1].y);
                 XB[t] = make_float4(Fx[2].x, Fx[2].y, Fx[3].x, Fx[3].y);
@@ -433,8 +445,8 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
                 XC[t] = make_float4(Fx[4].x, Fx[4].y, vel.x, vel.y);
             }
         }
-        pc1 = pc0;
-        pc0 = 2 - pc0;
+        s1 = s0;
+        s0 ^= 1;
         kr = ring_next<KP>(kr);
         par ^= (kr == 0) ? 1 : 0;
         ku = ring_next<KP>(ku);
