@@ -295,8 +295,8 @@ static int alloc_buffers(fvm_handle *h, int nx, int ny) {
     CKA(cudaMalloc(&h->mask, (size_t)g.plane));
     CK(cudaMemsetAsync(h->ct, 0, (size_t)nx * ny, h->stream));
     h->diag_parts = diagnostics_parts(g);
-    CKA(cudaMalloc(&h->d_diag, (size_t)(h->diag_parts * 8 + 16) * sizeof(double)));
-    h->bytes = state_bytes * NBUF + (size_t)g.plane * 5 + (size_t)nx * ny + (size_t)(h->diag_parts * 8 + 16) * 8;
+    CKA(cudaMalloc(&h->d_diag, (size_t)h->diag_parts * 8 * sizeof(double)));
+    h->bytes = state_bytes * NBUF + (size_t)g.plane * 5 + (size_t)nx * ny + (size_t)h->diag_parts * 8 * 8;
     h->tune = pick_tune(h, nx, ny);
     return FVM_OK;
 }
@@ -407,12 +407,15 @@ extern "C" int fvm_create(fvm_handle **out) {
     if (cudaMalloc(&h->sc, sizeof(DevScalars)) != cudaSuccess || cudaMalloc(&h->d_count, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&h->d_tmp, 16) != cudaSuccess || cudaMalloc(&h->d_counter, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&h->d_disp, sizeof(DisplayDesc)) != cudaSuccess ||
-        cudaMallocHost(&h->h_sc, sizeof(DevScalars)) != cudaSuccess) {
+        cudaMallocHost(&h->h_sc, sizeof(DevScalars) + 8 * sizeof(double)) != cudaSuccess) {
         delete h;
         return set_err(FVM_ERR_ALLOC, "fvm_create: allocation failed");
     }
+    static_assert(sizeof(DevScalars) % alignof(double) == 0, "the results follow the mirror");
+    h->h_res = reinterpret_cast<double *>(h->h_sc + 1);
     cudaMemsetAsync(h->sc, 0, sizeof(DevScalars), h->stream);
     cudaMemsetAsync(h->d_disp, 0, sizeof(DisplayDesc), h->stream);
+    cudaMemsetAsync(h->d_tmp, 0, 16, h->stream);
     cudaStreamSynchronize(h->stream);
     *out = h;
     return FVM_OK;
@@ -823,7 +826,7 @@ extern "C" int fvm_synchronize(fvm_handle *h) {
 static int cfl_maxima(fvm_handle *h, float *ms, float *mn) {
     if (!h->cfl_valid) {
         CK(launch_cfl_state(h->g, h->Un, h->mask, h->sc, h->stream));
-        h->launches += 2;
+        h->launches++;
         h->cfl_valid = true;
     }
     CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
@@ -858,7 +861,7 @@ extern "C" int fvm_queue_dt(fvm_handle *h, const fvm_sim_params *p) {
     if (!p) return set_err(FVM_ERR_INVALID, "null params");
     if (!h->cfl_valid) {
         CK(launch_cfl_state(h->g, h->Un, h->mask, h->sc, h->stream));
-        h->launches += 2;
+        h->launches++;
         h->cfl_valid = true;
     }
     CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
@@ -1025,11 +1028,11 @@ extern "C" int fvm_vector_arrows(fvm_handle *h, float *dev_vertex_data, int max_
 static int max_reduce(fvm_handle *h, int what, float *out) {
     CHECK_INIT(h);
     if (!out) return set_err(FVM_ERR_INVALID, "null output");
-    CK(cudaMemsetAsync(h->d_tmp, 0, sizeof(float), h->stream));
-    CK(launch_max_reduce(what, h->g, h->Un, h->d_tmp, h->stream));
+    float *res = reinterpret_cast<float *>(h->h_res);
+    CK(launch_max_reduce(what, h->g, h->Un, h->d_tmp, res, h->stream));
     h->launches++;
-    CK(cudaMemcpyAsync(out, h->d_tmp, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    *out = *res;
     return FVM_OK;
 }
 extern "C" int fvm_max_temperature(fvm_handle *h, float *out) { return max_reduce(h, 0, out); }
@@ -1051,12 +1054,11 @@ extern "C" int fvm_gpu_mem_info(size_t *free_bytes, size_t *total_bytes) {
 extern "C" int fvm_diagnostics(fvm_handle *h, fvm_diag *out) {
     CHECK_INIT(h);
     if (!out) return set_err(FVM_ERR_INVALID, "null output");
-    double *parts = h->d_diag, *fin = h->d_diag + (size_t)h->diag_parts * 8;
-    CK(launch_diagnostics(h->g, h->Un, h->ct, h->mask, h->prm.enable_viscosity ? 1 : 0, h->ext.prandtl,
-                          h->ext.prandtl == PRANDTL_REF, parts, h->diag_parts, fin, h->stream));
-    h->launches += 2;
-    double r[8];
-    CK(cudaMemcpyAsync(r, fin, sizeof r, cudaMemcpyDeviceToHost, h->stream));
+    const double *r = h->h_res;
+    CK(launch_diagnostics(h->g, h->Un, h->mask, h->prm.enable_viscosity ? 1 : 0, h->ext.prandtl,
+                          h->ext.prandtl == PRANDTL_REF, h->d_diag, h->diag_parts,
+                          reinterpret_cast<unsigned *>(h->d_tmp + 2), h->h_res, h->stream));
+    h->launches++;
     CK(cudaStreamSynchronize(h->stream));
     memset(out, 0, sizeof(*out));
     out->force_x = r[0];
@@ -1085,11 +1087,10 @@ extern "C" int fvm_shock_standoff(fvm_handle *h, double *standoff_out) {
         return FVM_OK;
     }
     const double p2 = pinf * (1.0 + 2.0 * g / (g + 1.0) * (M * M - 1.0));
-    double *dout = h->d_diag + (size_t)h->diag_parts * 8 + 8;
-    CK(launch_standoff(h->g, h->Un, h->sdf, pinf + 0.5 * (p2 - pinf), dout, h->stream));
+    CK(launch_standoff(h->g, h->Un, h->sdf, pinf + 0.5 * (p2 - pinf), h->h_res, h->stream));
     h->launches++;
-    CK(cudaMemcpyAsync(standoff_out, dout, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    *standoff_out = h->h_res[0];
     return FVM_OK;
 }
 

@@ -1,7 +1,10 @@
 // fvm_aux.cu -- off-step kernels behind the reference's readback / statistics
 // API: derived fields into device buffers, max-temperature / max-Mach
 // reductions, velocity arrows, FP64 diagnostics and the shock standoff scan.
+#include <cstdint>
+
 #include "fvm_kernels.cuh"
+#include "fvm_quads.cuh"
 #include "fvm_tma.cuh"
 
 namespace fvm {
@@ -19,74 +22,167 @@ __global__ void k_primitives(GridDesc g, const float *U, float *u, float *v, flo
     if (T) T[d] = TT;
 }
 
-// Derived field into a dense nx*ny destination.
-__global__ void k_derived(int kind, GridDesc g, const float *U, float *dst) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    size_t c = (size_t)j * g.pitch + i, d = (size_t)j * g.nx + i;
-    dst[d] = derived_value(kind, U[c], U[g.plane + c], U[2 * g.plane + c], U[4 * g.plane + c]);
+// The planes a derived field reads (derived_value): the others stay zero.
+template <int KIND>
+struct DerivedIn {
+    float4 rho, ru, rv, re;
+    __device__ __forceinline__ DerivedIn(const GridDesc &g, const float *U, const Quad &q) {
+        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        rho = KIND != 1 ? load4(U, q) : z;
+        ru = KIND >= 3 ? load4(U + g.plane, q) : z;
+        rv = KIND >= 3 ? load4(U + 2 * g.plane, q) : z;
+        re = KIND != 2 && KIND != 3 ? load4(U + 4 * g.plane, q) : z;
+    }
+    __device__ __forceinline__ float value(int k) const {
+        return derived_value(KIND, lane4(rho, k), lane4(ru, k), lane4(rv, k), lane4(re, k));
+    }
+};
+
+// Derived field into a dense nx*ny destination: 8 (density, pressure) to 20
+// (Mach) bytes per cell, DRAM-bound.  One launch per kind, so that only the
+// planes the kind needs are read.  VEC: every group's destination is 16-byte
+// aligned (nx a multiple of 4 and dst aligned).  Measured at 8192x4096,
+// all four planes read a cell at a time -> this: density and pressure 135 -> 39
+// us, temperature 135 -> 53, speed 135 -> 72, Mach 135 -> 92 (7.3 TB/s).
+template <int KIND, bool VEC>
+__global__ void __launch_bounds__(256) k_derived(GridDesc g, const float *__restrict__ U, float *__restrict__ dst) {
+    const unsigned e = blockIdx.x * 256u + threadIdx.x;
+    if (e >= quads(g)) return;
+    const Quad q = quad_at(g, e);
+    const DerivedIn<KIND> in(g, U, q);
+    if (VEC) {
+        *reinterpret_cast<float4 *>(dst + q.d) = make_float4(in.value(0), in.value(1), in.value(2), in.value(3));
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (k < q.n) dst[q.d + k] = in.value(k);
+    }
+}
+
+// (1 - w) a + w b, rounded the same way in every kernel variant (an image's
+// bytes must not depend on it).
+__device__ __forceinline__ float lerp_texel(float w, float a, float b) {
+    return __fmaf_rn(w, b, __fmul_rn(1.0f - w, a));
 }
 
 // The renderer's field pass (FIELD_FRAGMENT_SHADER, src/renderer.cpp:47-77)
 // with one pixel per cell: SOLID and GHOST cells dark grey, others the
 // derived value normalised by (v - lo) / (hi - lo + 1e-4), clamped to [0, 1],
 // then looked up in the 256-entry colour table the way a linearly filtered,
-// edge-clamped 1-D texture samples it.  fmt 0: RGBA float, fmt 1: RGBA8.
-__global__ void k_colormap(int kind, GridDesc g, const float *U, const uint8_t *ct,
-                           const __grid_constant__ ColormapLUT lut, float lo, float hi, void *out, int fmt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    const size_t c = (size_t)j * g.pitch + i, d = (size_t)j * g.nx + i;
-    const uint8_t t = ct[d];
-    float r, gr, b;
-    if (t == CT_SOLID || t == CT_GHOST) {
-        r = gr = b = 0.3f;
-    } else {
-        const float v = derived_value(kind, U[c], U[g.plane + c], U[2 * g.plane + c], U[4 * g.plane + c]);
-        const float s = fminf(fmaxf((v - lo) / (hi - lo + 0.0001f), 0.0f), 1.0f);
-        const float u = s * 256.0f - 0.5f;
-        const float fl = floorf(u);
-        const float a = u - fl;
-        const int i0 = min(max((int)fl, 0), 255), i1 = min(max((int)fl + 1, 0), 255);
-        r = (1.0f - a) * lut.rgb[3 * i0] + a * lut.rgb[3 * i1];
-        gr = (1.0f - a) * lut.rgb[3 * i0 + 1] + a * lut.rgb[3 * i1 + 1];
-        b = (1.0f - a) * lut.rgb[3 * i0 + 2] + a * lut.rgb[3 * i1 + 2];
+// edge-clamped 1-D texture samples it.  FMT 0: RGBA float, 1: RGBA8.
+// The table sits in shared memory as pairs of neighbouring entries, so a
+// lookup is two 16-byte loads; indexed in the kernel's parameters (constant
+// memory), lanes with different colours were served one after the other.
+// Mach -> RGBA8 at 8192x4096: 214 us that way, 132 us here (21 B per cell, 5.3
+// TB/s).
+template <int KIND, int FMT, bool VEC>
+__global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__restrict__ U,
+                                                  const uint8_t *__restrict__ mask,
+                                                  const __grid_constant__ ColormapLUT lut, float lo, float hi,
+                                                  void *__restrict__ out) {
+    // entry i: {r_i, g_i, b_i, r_i+1}, {g_i+1, b_i+1, -, -}
+    __shared__ float4 ta[256];
+    __shared__ float2 tb[256];
+    {
+        const int i = threadIdx.x, n = min(i + 1, 255);
+        ta[i] = make_float4(lut.rgb[3 * i], lut.rgb[3 * i + 1], lut.rgb[3 * i + 2], lut.rgb[3 * n]);
+        tb[i] = make_float2(lut.rgb[3 * n + 1], lut.rgb[3 * n + 2]);
     }
-    if (fmt == 0) {
-        reinterpret_cast<float4 *>(out)[d] = make_float4(r, gr, b, 1.0f);
-    } else {
-        auto q = [](float x) { return (unsigned)__float2int_rn(fminf(fmaxf(x, 0.0f), 1.0f) * 255.0f); };
-        reinterpret_cast<uchar4 *>(out)[d] = make_uchar4(q(r), q(gr), q(b), 255);
-    }
-}
-
-// cellTypeToFloatKernel (src/solver.cu:3444-3450)
-__global__ void k_ct_to_float(long long n, const uint8_t *ct, float *dst) {
-    long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < n) dst[e] = static_cast<float>(ct[e]);
-}
-
-// what = 0: max temperature of the primitives (getMaxTemperature,
-// src/solver.cu:2835-2867); what = 1: max local Mach (computeMachNumberKernel,
-// src/solver.cu:2782-2794).  out_dev must be zeroed by the caller.
-__global__ void __launch_bounds__(256) k_max_reduce(int what, GridDesc g, const float *U, float *out_dev) {
-    float m = 0.0f;
-    const long long n = (long long)g.nx * g.ny;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(e / g.nx), i = (int)(e % g.nx);
-        const size_t c = (size_t)j * g.pitch + i;
-        float u, v, p, T;
-        const float rho = U[c];
-        prim_from_cons(rho, U[g.plane + c], U[2 * g.plane + c], U[3 * g.plane + c], U[4 * g.plane + c], u, v, p, T);
-        if (what == 0) {
-            m = fmaxf(m, T);
+    __syncthreads();
+    const unsigned total = quads(g);
+    for (unsigned e = blockIdx.x * 256u + threadIdx.x; e < total; e += gridDim.x * 256u) {
+        const Quad q = quad_at(g, e);
+        const DerivedIn<KIND> in(g, U, q);
+        const uint32_t m4 = __ldg(reinterpret_cast<const uint32_t *>(mask + q.c));
+        float4 px[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float r, gr, b;
+            if ((m4 >> (8 * k)) & MB_WALL) {
+                r = gr = b = 0.3f;
+            } else {
+                const float s = fminf(fmaxf((in.value(k) - lo) / (hi - lo + 0.0001f), 0.0f), 1.0f);
+                const float u = s * 256.0f - 0.5f;
+                const float fl = floorf(u);
+                const float w = u - fl;
+                // the texel pair (fl, fl + 1) clamped to the edge: below the
+                // first texel both are entry 0
+                const int i0 = min(max((int)fl, 0), 255);
+                const float4 A = ta[i0];
+                const float2 B = tb[i0];
+                const bool first = (int)fl < 0;
+                r = lerp_texel(w, A.x, first ? A.x : A.w);
+                gr = lerp_texel(w, A.y, first ? A.y : B.x);
+                b = lerp_texel(w, A.z, first ? A.z : B.y);
+            }
+            px[k] = make_float4(r, gr, b, 1.0f);
+        }
+        if (FMT == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < q.n) reinterpret_cast<float4 *>(out)[q.d + k] = px[k];
         } else {
-            float rho_val = rho + 1e-10f;
-            float speed = sqrtf(u * u + v * v);
-            float cs = sqrtf(GAMMA * p / rho_val);
-            m = fmaxf(m, speed / (cs + 1e-10f));
+            auto quant = [](float x) { return (unsigned)__float2int_rn(fminf(fmaxf(x, 0.0f), 1.0f) * 255.0f); };
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                w[k] = quant(px[k].x) | (quant(px[k].y) << 8) | (quant(px[k].z) << 16) | (255u << 24);
+            if (VEC) {
+                *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(out) + q.d) = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k < q.n) reinterpret_cast<uint32_t *>(out)[q.d + k] = w[k];
+            }
+        }
+    }
+}
+
+// cellTypeToFloatKernel (src/solver.cu:3444-3450); both arrays are dense, four
+// cells per thread where the destination is 16-byte aligned (VEC).
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_ct_to_float(long long n, const uint8_t *__restrict__ ct,
+                                                     float *__restrict__ dst) {
+    const long long e = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+    if (VEC && e + 4 <= n) {
+        const uchar4 c = *reinterpret_cast<const uchar4 *>(ct + e);
+        *reinterpret_cast<float4 *>(dst + e) =
+            make_float4(static_cast<float>(c.x), static_cast<float>(c.y), static_cast<float>(c.z), static_cast<float>(c.w));
+        return;
+    }
+    for (long long k = e; k < e + 4 && k < n; k++) dst[k] = static_cast<float>(ct[k]);
+}
+
+// WHAT = 0: max temperature of the primitives (getMaxTemperature,
+// src/solver.cu:2835-2867); WHAT = 1: max local Mach (computeMachNumberKernel,
+// src/solver.cu:2782-2794).  The last block writes the maximum to `out` in
+// pinned host memory and leaves the scratch {maximum, counter} zero for the
+// next call: no memset before and no copy after.  2048x1024: 12.4 us one cell at a time,
+// 10.0 us here.
+template <int WHAT>
+__global__ void __launch_bounds__(256, 6) k_max_reduce(GridDesc g, const float *__restrict__ U, float *scratch,
+                                                    float *out) {
+    float m = 0.0f;
+    const unsigned total = quads(g);
+    for (unsigned e = blockIdx.x * 256u + threadIdx.x; e < total; e += gridDim.x * 256u) {
+        const Quad q = quad_at(g, e);
+        const float4 R = load4(U, q), RU = load4(U + g.plane, q), RV = load4(U + 2 * g.plane, q),
+                     E = load4(U + 3 * g.plane, q), RE = load4(U + 4 * g.plane, q);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float u, v, p, T;
+            const float rho = lane4(R, k);
+            prim_from_cons(rho, lane4(RU, k), lane4(RV, k), lane4(E, k), lane4(RE, k), u, v, p, T);
+            float x;
+            if (WHAT == 0) {
+                x = T;
+            } else {
+                float rho_val = rho + 1e-10f;
+                float speed = sqrtf(u * u + v * v);
+                float cs = sqrtf(GAMMA * p / rho_val);
+                x = speed / (cs + 1e-10f);
+            }
+            if (k < q.n) m = fmaxf(m, x);
         }
     }
     __shared__ float ws[8];
@@ -96,7 +192,11 @@ __global__ void __launch_bounds__(256) k_max_reduce(int what, GridDesc g, const 
     if (threadIdx.x == 0) {
         float mm = 0.0f;
         for (int k = 0; k < 8; k++) mm = fmaxf(mm, ws[k]);
-        atomic_max_nonneg(out_dev, mm);
+        atomic_max_nonneg(scratch, mm);
+    }
+    if (last_block(reinterpret_cast<unsigned *>(scratch + 1)) && threadIdx.x == 0) {
+        *out = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(scratch), 0u));
+        __threadfence_system();
     }
 }
 
@@ -151,7 +251,7 @@ __global__ void k_arrows(GridDesc g, const float *U, float *vertexData, int *cou
 // force on the obstacle is (-p_face n + tau.n) dA, n the unit normal from the
 // wall cell to the fluid cell, p_face the pressure of the left/bottom cell
 // (the reference's wall-face flux, src/solver.cu:1594,1679), tau and q at the
-// fluid cell.  Per-CTA partials then one ordered final sum: deterministic.
+// fluid cell.  Deterministic: the sums' order depends on the grid alone.
 constexpr int kDiag = 8;  // fx, fy, mass, mx, my, E, heat, heat_max
 
 struct DiagCtx {
@@ -179,101 +279,194 @@ __device__ void stress_at(const DiagCtx &d, int i, int j, float out[5]) {
                 d.va, out);
 }
 
-__global__ void __launch_bounds__(256) k_diag_partial(DiagCtx d, int viscous, double *partials) {
+// The wall face between cell (i, j) and its right (dir 0) or upper (dir 1)
+// neighbour; wa: (i, j) is the wall.
+__device__ __forceinline__ void diag_face(const DiagCtx &d, int i, int j, int dir, bool wa, int viscous,
+                                          double acc[kDiag]) {
+    const double sgn = wa ? 1.0 : -1.0;
+    const int fi = wa ? (dir == 0 ? i + 1 : i) : i;
+    const int fj = wa ? (dir == 0 ? j : j + 1) : j;
+    const double dA = dir == 0 ? (double)d.g.dy : (double)d.g.dx;
+    const double nxn = dir == 0 ? sgn : 0.0, nyn = dir == 1 ? sgn : 0.0;
+    float u, v, p, T;
+    prim_at(d, i, j, u, v, p, T);
+    double fx = -(double)p * nxn * dA, fy = -(double)p * nyn * dA;
+    if (viscous) {
+        float t5[5];
+        stress_at(d, fi, fj, t5);
+        fx += ((double)t5[0] * nxn + (double)t5[2] * nyn) * dA;
+        fy += ((double)t5[2] * nxn + (double)t5[1] * nyn) * dA;
+        const double qw = -((double)t5[3] * nxn + (double)t5[4] * nyn);
+        acc[6] += qw * dA;
+        acc[7] = fmax(acc[7], qw);
+    }
+    acc[0] += fx;
+    acc[1] += fy;
+}
+
+__device__ __forceinline__ double diag_combine(int k, double a, double b) { return k == 7 ? fmax(a, b) : a + b; }
+
+// Per-block partials, then the last block to finish sums them in a fixed
+// order (one warp per quantity, lane l the partials l, l+32, ..., then a
+// shuffle tree), so the result does not depend on which block that is; it
+// goes straight to pinned host memory.  Reads 16 B of state and 1 B of mask
+// per cell: the loads of a group of four cells are issued together and the
+// walls are found four cells at a time on the mask words.  A wall face costs
+// some 30 scattered loads; each warp lists its faces in shared memory (in the
+// order of its cells) and works them off 32 at a time, one per lane, instead
+// of one lane after another for the faces its own cells have.  2048x1024:
+// 18 us; one cell per thread with a second kernel in which one thread summed
+// the partials took 36 + 160 us, faces in their cells' lanes 33 us.
+constexpr int kFaceList = 32 + 256;  // less than a round left over, plus all faces of 32 groups
+__global__ void __launch_bounds__(256, 4) k_diagnostics(DiagCtx d, int viscous, double *partials, unsigned *counter,
+                                                     double *out) {
+    __shared__ unsigned long long faces[8][kFaceList];  // group index * 8 + face of the group: k (x-faces), 4 + k (y-faces)
     double acc[kDiag];
+#pragma unroll
     for (int k = 0; k < kDiag; k++) acc[k] = 0.0;
     const GridDesc g = d.g;
-    const long long n = (long long)g.nx * g.ny;
-    const double dxd = g.dx, dyd = g.dy, area = dxd * dyd;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(e / g.nx), i = (int)(e % g.nx);
-        const size_t c = (size_t)j * g.pitch + i;
-        const bool wa = (d.mask[c] & MB_WALL) != 0;
-        if (!wa) {
-            acc[2] += (double)d.U[c] * area;
-            acc[3] += (double)d.U[g.plane + c] * area;
-            acc[4] += (double)d.U[2 * g.plane + c] * area;
-            acc[5] += (double)d.U[3 * g.plane + c] * area;
+    const unsigned total = quads(g);
+    constexpr uint32_t W4 = MB_WALL * 0x01010101u;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned long long *list = faces[warp];
+    int listed = 0;
+    // one listed face per lane
+    auto work = [&](int at, bool mine) {
+        __syncwarp();
+        if (mine) {
+            const unsigned long long code = list[at];
+            const Quad q = quad_at(g, (unsigned)(code >> 3));
+            const int i = q.i + (int)(code & 3u), dir = (int)(code >> 2) & 1;
+            diag_face(d, i, q.j, dir, (d.mask[(size_t)q.j * g.pitch + i] & MB_WALL) != 0, viscous, acc);
         }
-        for (int dir = 0; dir < 2; dir++) {
-            if (dir == 0 && i >= g.nx - 1) continue;
-            if (dir == 1 && j >= g.ny - 1) continue;
-            const size_t b = dir == 0 ? c + 1 : c + g.pitch;
-            const bool wb = (d.mask[b] & MB_WALL) != 0;
-            if (wa == wb) continue;
-            const double sgn = wa ? 1.0 : -1.0;
-            const int fi = wa ? (dir == 0 ? i + 1 : i) : i;
-            const int fj = wa ? (dir == 0 ? j : j + 1) : j;
-            const double dA = dir == 0 ? dyd : dxd;
-            const double nxn = dir == 0 ? sgn : 0.0, nyn = dir == 1 ? sgn : 0.0;
-            float u, v, p, T;
-            prim_at(d, i, j, u, v, p, T);
-            double fx = -(double)p * nxn * dA, fy = -(double)p * nyn * dA;
-            if (viscous) {
-                float t5[5];
-                stress_at(d, fi, fj, t5);
-                fx += ((double)t5[0] * nxn + (double)t5[2] * nyn) * dA;
-                fy += ((double)t5[2] * nxn + (double)t5[1] * nyn) * dA;
-                const double qw = -((double)t5[3] * nxn + (double)t5[4] * nyn);
-                acc[6] += qw * dA;
-                acc[7] = fmax(acc[7], qw);
+        __syncwarp();
+    };
+    for (unsigned e0 = blockIdx.x * 256u + 32u * warp; e0 < total; e0 += gridDim.x * 256u) {
+        const unsigned e = e0 + lane;
+        uint32_t bits = 0u;
+        if (e < total) {
+            const Quad q = quad_at(g, e);
+            const uint8_t *mrow = d.mask + q.c;
+            const float4 R = load4(d.U, q), RU = load4(d.U + g.plane, q), RV = load4(d.U + 2 * g.plane, q),
+                         E = load4(d.U + 3 * g.plane, q);
+            const bool top = q.j >= g.ny - 1, right = q.i + 4 >= g.nx;
+            const uint32_t m = __ldg(reinterpret_cast<const uint32_t *>(mrow)) & W4;
+            const uint32_t up = __ldg(reinterpret_cast<const uint32_t *>(top ? mrow : mrow + g.pitch)) & W4;
+            const uint32_t next = right ? 0u : (uint32_t)__ldg(mrow + 4) & MB_WALL;
+            // cells of the group inside the grid; a last column has no right neighbour
+            const uint32_t in = W4 >> (8 * (4 - q.n));
+            const uint32_t inx = right ? in >> 8 : in;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if ((in & ~m) >> (8 * k) & MB_WALL) {
+                    acc[2] += (double)lane4(R, k);
+                    acc[3] += (double)lane4(RU, k);
+                    acc[4] += (double)lane4(RV, k);
+                    acc[5] += (double)lane4(E, k);
+                }
             }
-            acc[0] += fx;
-            acc[1] += fy;
+            const uint32_t fx = (m ^ ((m >> 8) | (next << 24))) & inx, fy = (m ^ up) & in;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                bits |= ((fx >> (8 * k)) & 1u) << k | ((fy >> (8 * k)) & 1u) << (4 + k);
+        }
+        if (__any_sync(0xffffffffu, bits != 0u)) {
+            int before = __popc(bits);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += y;
+            }
+            const int added = __shfl_sync(0xffffffffu, before, 31);
+            int at = listed + before - __popc(bits);
+            for (uint32_t b = bits; b; b &= b - 1u) list[at++] = (unsigned long long)e * 8u + (unsigned)(__ffs(b) - 1);
+            for (listed += added; listed >= 32; listed -= 32) work(listed - 32 + lane, true);
+            __syncwarp();
         }
     }
-    __shared__ double s[kDiag][256];
-    for (int k = 0; k < kDiag; k++) s[k][threadIdx.x] = acc[k];
+    work(lane, lane < listed);
+    const double area = (double)g.dx * (double)g.dy;
+#pragma unroll
+    for (int k = 2; k < 6; k++) acc[k] *= area;
+    __shared__ double s[8][kDiag];
+#pragma unroll
+    for (int k = 0; k < kDiag; k++) {
+        double x = acc[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = diag_combine(k, x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (lane == 0) s[warp][k] = x;
+    }
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int k = 0; k < kDiag; k++)
-                s[k][threadIdx.x] = (k == 7) ? fmax(s[k][threadIdx.x], s[k][threadIdx.x + w])
-                                             : s[k][threadIdx.x] + s[k][threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x < kDiag) {
+        double x = s[0][threadIdx.x];
+        for (int w = 1; w < 8; w++) x = diag_combine(threadIdx.x, x, s[w][threadIdx.x]);
+        partials[(size_t)blockIdx.x * kDiag + threadIdx.x] = x;
     }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < kDiag; k++) partials[(size_t)blockIdx.x * kDiag + k] = s[k][0];
+    if (!last_block(counter)) return;
+    static_assert(kDiag == 8, "one warp per quantity");
+    double x = 0.0;
+    for (unsigned b = lane; b < gridDim.x; b += 32)
+        x = diag_combine(warp, x, __ldcg(&partials[(size_t)b * kDiag + warp]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = diag_combine(warp, x, __shfl_xor_sync(0xffffffffu, x, o));
+    if (lane == 0) {
+        out[warp] = x;
+        __threadfence_system();
+    }
 }
 
-__global__ void k_diag_final(const double *partials, int nparts, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double acc[kDiag];
-    for (int k = 0; k < kDiag; k++) acc[k] = 0.0;
-    for (int b = 0; b < nparts; b++)
-        for (int k = 0; k < kDiag; k++)
-            acc[k] = (k == 7) ? fmax(acc[k], partials[(size_t)b * kDiag + k]) : acc[k] + partials[(size_t)b * kDiag + k];
-    for (int k = 0; k < kDiag; k++) out[k] = acc[k];
+// Smallest index found by the block's threads (INT_MAX: none).
+__device__ __forceinline__ int block_min_index(int x) {
+    __shared__ int first;
+    if (threadIdx.x == 0) first = 0x7fffffff;
+    __syncthreads();
+    x = __reduce_min_sync(0xffffffffu, x);
+    if ((threadIdx.x & 31) == 0 && x != 0x7fffffff) atomicMin(&first, x);
+    __syncthreads();
+    const int r = first;
+    __syncthreads();
+    return r;
 }
 
-// Shock standoff along row ny/2 (see fvm_b200.h); one thread scans the row.
-__global__ void k_standoff(GridDesc g, const float *U, const float *sdf, double p_mid, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int j = g.ny / 2;
+// Shock standoff along row ny/2 (see fvm_b200.h): the first downward zero of
+// the distance field, then the first upward crossing of p_mid before it.  One
+// block looks at 1024 cells at a time and stops at the first hit (one thread
+// scanning the row paid a load's latency per cell: 80 us at 2048x1024, 5 us
+// here).  The result goes to pinned host memory.
+__global__ void __launch_bounds__(1024) k_standoff(GridDesc g, const float *U, const float *sdf, double p_mid,
+                                                   double *out) {
+    const size_t row = (size_t)(g.ny / 2) * g.pitch;
     const double dxd = g.dx;
-    int ib = -1;
-    double xb = 0.0;
-    for (int i = 0; i + 1 < g.nx; i++) {
-        double a = sdf[(size_t)j * g.pitch + i], b = sdf[(size_t)j * g.pitch + i + 1];
-        if (a > 0 && b <= 0) {
-            xb = (i + 0.5) * dxd + dxd * a / (a - b);
-            ib = i;
-            break;
+    int ib = 0x7fffffff;
+    for (int i0 = 0; i0 + 1 < g.nx && ib == 0x7fffffff; i0 += 1024) {
+        const int i = i0 + (int)threadIdx.x;
+        const bool hit = i + 1 < g.nx && sdf[row + i] > 0.0f && sdf[row + i + 1] <= 0.0f;
+        ib = block_min_index(hit ? i : 0x7fffffff);
+    }
+    int is = 0x7fffffff;
+    if (ib != 0x7fffffff) {
+        auto pressure = [&](int i) {
+            const size_t c = row + i;
+            float u, v, p, T;
+            prim_from_cons(U[c], U[g.plane + c], U[2 * g.plane + c], U[3 * g.plane + c], U[4 * g.plane + c], u, v, p, T);
+            return (double)p;
+        };
+        for (int i0 = 1; i0 <= ib && is == 0x7fffffff; i0 += 1024) {
+            const int i = i0 + (int)threadIdx.x;
+            const bool hit = i <= ib && pressure(i - 1) < p_mid && pressure(i) >= p_mid;
+            is = block_min_index(hit ? i : 0x7fffffff);
+        }
+        if (threadIdx.x == 0 && is != 0x7fffffff) {
+            const double a = sdf[row + ib], b = sdf[row + ib + 1];
+            const double xb = (ib + 0.5) * dxd + dxd * a / (a - b);
+            const double p0 = pressure(is - 1), p1 = pressure(is);
+            const double xs = (is - 1 + 0.5) * dxd + dxd * (p_mid - p0) / (p1 - p0);
+            *out = xb - xs;
         }
     }
-    *out = __longlong_as_double(0x7ff8000000000000ULL);
-    if (ib < 0) return;
-    float pprev = 0.0f;
-    for (int i = 0; i <= ib; i++) {
-        size_t c = (size_t)j * g.pitch + i;
-        float u, v, p, T;
-        prim_from_cons(U[c], U[g.plane + c], U[2 * g.plane + c], U[3 * g.plane + c], U[4 * g.plane + c], u, v, p, T);
-        if (i > 0 && (double)pprev < p_mid && (double)p >= p_mid) {
-            double xs = (i - 1 + 0.5) * dxd + dxd * (p_mid - (double)pprev) / ((double)p - (double)pprev);
-            *out = xb - xs;
-            return;
-        }
-        pprev = p;
+    if (threadIdx.x == 0) {
+        if (is == 0x7fffffff) *out = __longlong_as_double(0x7ff8000000000000ULL);
+        __threadfence_system();
     }
 }
 
@@ -287,30 +480,73 @@ cudaError_t launch_primitives(const GridDesc &g, const float *U, float *u, float
     return cudaGetLastError();
 }
 
-cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *ct, const ColormapLUT &lut,
+// whether every group of four cells of a dense nx*ny array of `elem`-byte
+// cells starts on a 16-byte boundary when four cells are 16 bytes
+static bool dense_aligned(const GridDesc &g, const void *p) {
+    return (g.nx & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+}
+
+template <int KIND>
+static void colormap_k(const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut, float lo,
+                       float hi, void *out, int fmt, cudaStream_t st) {
+    // enough blocks to fill the chip several times over, each filling its table once
+    const unsigned nb = quad_blocks(g, 148 * 32);
+    if (fmt == 0)
+        k_colormap<KIND, 0, false><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
+    else if (dense_aligned(g, out))
+        k_colormap<KIND, 1, true><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
+    else
+        k_colormap<KIND, 1, false><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
+}
+
+cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut,
                             float lo, float hi, void *out, int fmt, cudaStream_t st) {
-    dim3 b(32, 8);
-    k_colormap<<<grid2d(g, b), b, 0, st>>>(kind, g, U, ct, lut, lo, hi, out, fmt);
+    switch (kind) {
+    case 0: colormap_k<0>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    case 1: colormap_k<1>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    case 2: colormap_k<2>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    case 3: colormap_k<3>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    default: colormap_k<4>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    }
     return cudaGetLastError();
 }
 
+template <int KIND>
+static void derived_k(const GridDesc &g, const float *U, float *dst, cudaStream_t st) {
+    if (dense_aligned(g, dst))
+        k_derived<KIND, true><<<quad_blocks(g), 256, 0, st>>>(g, U, dst);
+    else
+        k_derived<KIND, false><<<quad_blocks(g), 256, 0, st>>>(g, U, dst);
+}
+
 cudaError_t launch_derived(int kind, const GridDesc &g, const float *U, float *dst, cudaStream_t st) {
-    dim3 b(32, 8);
-    k_derived<<<grid2d(g, b), b, 0, st>>>(kind, g, U, dst);
+    switch (kind) {
+    case 0: derived_k<0>(g, U, dst, st); break;
+    case 1: derived_k<1>(g, U, dst, st); break;
+    case 2: derived_k<2>(g, U, dst, st); break;
+    case 3: derived_k<3>(g, U, dst, st); break;
+    default: derived_k<4>(g, U, dst, st); break;
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_ct_to_float(const GridDesc &g, const uint8_t *ct, float *dst, cudaStream_t st) {
-    long long n = (long long)g.nx * g.ny;
-    k_ct_to_float<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, ct, dst);
+    const long long n = (long long)g.nx * g.ny;
+    const unsigned nb = (unsigned)((n + 1023) / 1024);
+    if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)
+        k_ct_to_float<true><<<nb, 256, 0, st>>>(n, ct, dst);
+    else
+        k_ct_to_float<false><<<nb, 256, 0, st>>>(n, ct, dst);
     return cudaGetLastError();
 }
 
-cudaError_t launch_max_reduce(int what, const GridDesc &g, const float *U, float *out_dev, cudaStream_t st) {
-    long long n = (long long)g.nx * g.ny;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    k_max_reduce<<<blocks, 256, 0, st>>>(what, g, U, out_dev);
+cudaError_t launch_max_reduce(int what, const GridDesc &g, const float *U, float *scratch, float *out_host,
+                              cudaStream_t st) {
+    const unsigned nb = quad_blocks(g, 148 * 6);  // one resident wave
+    if (what == 0)
+        k_max_reduce<0><<<nb, 256, 0, st>>>(g, U, scratch, out_host);
+    else
+        k_max_reduce<1><<<nb, 256, 0, st>>>(g, U, scratch, out_host);
     return cudaGetLastError();
 }
 
@@ -322,29 +558,23 @@ cudaError_t launch_arrows_cap(const GridDesc &g, const float *U, float *vertex, 
     return cudaGetLastError();
 }
 
-int diagnostics_parts(const GridDesc &g) {
-    long long n = (long long)g.nx * g.ny;
-    long long b = (n + 255) / 256;
-    return (int)(b < 592 ? b : 592);
-}
+int diagnostics_parts(const GridDesc &g) { return (int)quad_blocks(g, 592); }
 
-cudaError_t launch_diagnostics(const GridDesc &g, const float *U, const uint8_t *ct, const uint8_t *mask, int viscous,
-                               float prandtl, int ref_prandtl, double *partials, int nparts, double *out8,
+cudaError_t launch_diagnostics(const GridDesc &g, const float *U, const uint8_t *mask, int viscous, float prandtl,
+                               int ref_prandtl, double *partials, int nparts, unsigned *counter, double *out_host,
                                cudaStream_t st) {
-    (void)ct;
     DiagCtx d;
     d.g = g;
     d.U = U;
     d.mask = mask;
     d.va = viscous_args(g.dx, g.dy, prandtl, ref_prandtl != 0);
-    k_diag_partial<<<nparts, 256, 0, st>>>(d, viscous, partials);
-    k_diag_final<<<1, 32, 0, st>>>(partials, nparts, out8);
+    k_diagnostics<<<nparts, 256, 0, st>>>(d, viscous, partials, counter, out_host);
     return cudaGetLastError();
 }
 
-cudaError_t launch_standoff(const GridDesc &g, const float *U, const float *sdf, double p_mid, double *out,
+cudaError_t launch_standoff(const GridDesc &g, const float *U, const float *sdf, double p_mid, double *out_host,
                             cudaStream_t st) {
-    k_standoff<<<1, 32, 0, st>>>(g, U, sdf, p_mid, out);
+    k_standoff<<<1, 1024, 0, st>>>(g, U, sdf, p_mid, out_host);
     return cudaGetLastError();
 }
 

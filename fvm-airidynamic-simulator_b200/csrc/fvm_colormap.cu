@@ -81,7 +81,7 @@ extern "C" int fvm_colormap_to_device(fvm_handle *h, int field_kind, int colorma
         return fvm_internal_set_error(FVM_ERR_INVALID, "fvm_colormap_to_device: unknown pixel format");
     ColormapLUT L;
     build_lut(colormap, L);
-    cudaError_t e = launch_colormap(field_kind, h->g, h->Un, h->ct, L, min_val, max_val, dev_rgba, format, h->stream);
+    cudaError_t e = launch_colormap(field_kind, h->g, h->Un, h->mask, L, min_val, max_val, dev_rgba, format, h->stream);
     if (e != cudaSuccess) return fvm_internal_set_error(FVM_ERR_CUDA, cudaGetErrorString(e));
     h->launches++;
     return FVM_OK;

@@ -39,9 +39,10 @@ struct fvm_handle {
     int *d_count = nullptr;
     DevScalars *sc = nullptr;
     DevScalars *h_sc = nullptr;  // pinned mirror
-    float *d_tmp = nullptr;      // reduction scratch (1 float)
+    float *d_tmp = nullptr;      // reduction scratch: {maximum, counter} of the max pass, counter of the diagnostics
+    double *h_res = nullptr;     // 8 results the reduction kernels write to the host (behind h_sc, pinned)
     int *d_counter = nullptr;    // arrows counter
-    double *d_diag = nullptr;    // partials + 8 finals + standoff
+    double *d_diag = nullptr;    // partials of the diagnostics
     int diag_parts = 0;
     StageTune tune{128, 6, 32};
     bool dt_ready = false;       // recompute policy: sc->dt holds the next dt

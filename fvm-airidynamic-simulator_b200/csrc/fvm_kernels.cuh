@@ -51,7 +51,7 @@ cudaError_t launch_wait_probe(DevScalars *sc, long long limit_cycles, cudaStream
 // Phase-1 boundary conditions in place on a whole state (set-up path).
 cudaError_t launch_bc_phase1(const GridDesc &g, float *U, const uint8_t *mask, const Freestream &fs, cudaStream_t st);
 // CFL maxima of a state (speed over all cells; nu = mu(T)/rho, mu = 0 in solids),
-// accumulated into sc->red, then published to sc->cfl by a one-block finalize.
+// published to sc->cfl by the last block (sc->red and sc->counter are zero before and after).
 cudaError_t launch_cfl_state(const GridDesc &g, const float *U, const uint8_t *mask, DevScalars *sc, cudaStream_t st);
 // Set the dynamic shared-memory attribute of every step kernel of a tuning.
 cudaError_t prepare_step_kernels(const StageTune &tn);
@@ -70,17 +70,22 @@ cudaError_t launch_derived(int kind, const GridDesc &g, const float *U, float *d
 struct ColormapLUT {
     float rgb[256 * 3];
 };
-cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *ct, const ColormapLUT &lut,
+// mask: the pitched mask bytes (their wall bit marks SOLID and GHOST cells)
+cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut,
                             float lo, float hi, void *out, int fmt, cudaStream_t st);
 cudaError_t launch_ct_to_float(const GridDesc &g, const uint8_t *ct, float *dst, cudaStream_t st);
-cudaError_t launch_max_reduce(int what, const GridDesc &g, const float *U, float *out_dev, cudaStream_t st);
+// The results of the next three go to pinned host memory (out_host), valid once
+// the stream is synchronized; `scratch` / `counter` (8 / 4 bytes of device
+// memory) are zero before and after.
+cudaError_t launch_max_reduce(int what, const GridDesc &g, const float *U, float *scratch, float *out_host,
+                              cudaStream_t st);
 cudaError_t launch_arrows_cap(const GridDesc &g, const float *U, float *vertex, int cap, int *counter, int step,
                               float u_inf, float max_len, float head_angle, float head_len, cudaStream_t st);
-cudaError_t launch_diagnostics(const GridDesc &g, const float *U, const uint8_t *ct, const uint8_t *mask,
-                               int viscous, float prandtl, int ref_prandtl, double *partials, int nparts,
-                               double *out8, cudaStream_t st);
+cudaError_t launch_diagnostics(const GridDesc &g, const float *U, const uint8_t *mask, int viscous, float prandtl,
+                               int ref_prandtl, double *partials, int nparts, unsigned *counter, double *out_host,
+                               cudaStream_t st);
 int diagnostics_parts(const GridDesc &g);
-cudaError_t launch_standoff(const GridDesc &g, const float *U, const float *sdf, double p_mid, double *out,
+cudaError_t launch_standoff(const GridDesc &g, const float *U, const float *sdf, double p_mid, double *out_host,
                             cudaStream_t st);
 
 }  // namespace fvm
