@@ -238,28 +238,46 @@ struct TuneKey {
 };
 static std::map<TuneKey, StageTune> g_tune_cache;
 
-// Default launch shape before (or without) autotuning: 128 threads, a 4-row
-// input ring and about 48 row bands: the tile height in {4, 8, 16, ..., 64}
-// nearest ny / 48.  Measured on B200 (NS step): 1024x512 fastest at 8 rows
-// (0.071 ms; 10 and 12 rows 0.080 / 0.077), 2048x1024 at 24 (0.181 ms; 32 rows
-// 0.197), 4096x2048 at 40-48 (0.614 ms; 64 rows 0.661), 8192x4096 at 64;
-// 512x256 wants 4.  Small grids are latency-bound and want many short tiles,
-// large ones tall tiles, which keep the per-tile halo rows cheap.
-static StageTune heuristic_tune(int, int ny) {
-    StageTune t{128, 4, 4};
-    const double want = ny / 48.0;
-    double best = 1e30;
-    for (int rows : {4, 8, 16, 24, 32, 40, 48, 56, 64}) {
-        const double d = rows > want ? rows - want : want - rows;
-        if (d < best) {
-            best = d;
-            t.rows = rows;
-        }
-    }
-    return t;
+// Rows per CTA of a marching kernel that keeps `slots` CTAs resident.  If the
+// whole grid fits into one resident wave with tiles of at most 24 rows, the
+// shortest such tiles: every CTA starts at once and none is left for a second,
+// nearly empty wave.  Else about 96 row bands, or 64 from 2000 rows up: several
+// waves, which the block scheduler evens out, of tiles tall enough to keep the
+// halo rows cheap (the more waves, the taller).
+// Measured on B200, step in us by rows: Euler 2048x1024 (one wave from 20)
+// 16: 127, 20: 117, 24: 131; 2400x1200 12: 159, 24: 166; 3000x1500 16: 225, 32:
+// 231; NS 3000x1500 16: 334, 32: 341; 4096x2048 20: 578, 32: 573, 64: 632;
+// 6000x3000 24: 1150, 40: 1128; 8192x4096 40: 2036, 64: 2020.
+static int march_rows(int nx, int ny, int slots) {
+    const int strips = (nx + 123) / 124;
+    for (int rows = 4; rows <= 24; rows += 4)
+        if ((long long)strips * ((ny + rows - 1) / rows) <= slots) return rows;
+    const double want = ny / (ny < 2000 ? 96.0 : 64.0);
+    int best = 12;
+    for (int rows : {16, 20, 24, 32, 40, 48, 64})
+        if (std::abs(rows - want) < std::abs(best - want)) best = rows;
+    return best;
 }
 
-static StageTune pick_tune(const fvm_handle *h, int nx, int ny);
+// Default launch shape before (or without) autotuning: marching kernels of 128
+// threads with a 4-row input ring, and the flat stage kernel up to 1.5 million
+// cells.  There a marching stage leaves the chip mostly idle: a CTA works
+// through its row pairs one after another (2 us each, the latency of one
+// pair's dependent arithmetic) and taller tiles mean fewer CTAs, while the flat
+// kernel has a thread for every face at once; above, the flat kernel's
+// two-cell halo (1.6 times the cells of a 32x14 tile) costs more than that.
+// Measured Euler steps, marching (best rows) -> flat, us: 256x128 22.6 -> 16.4,
+// 512x256 27.3 -> 20.6, 1024x512 49.2 -> 40.0, 1501x777 77.3 -> 72.7, 1800x900
+// 96.6 -> 98.8, 2048x1024 116.9 -> 123.7.  Tiles of 32x14 cells, or of 32x6
+// while the taller ones would give fewer than 3 CTAs per SM (512x256 20.6
+// against 22.6 us, 640x320 25.7 either way, 1024x512 44.0 against 40.0).
+static StageTune heuristic_tune(int nx, int ny) {
+    constexpr int kSms = 148;
+    // 6 stage CTAs and 5 viscous CTAs of 128 threads per SM
+    StageTune t{128, 4, march_rows(nx, ny, 6 * kSms), march_rows(nx, ny, 5 * kSms), 0};
+    if ((long long)nx * ny <= 1500000) t.flat_pairs = (long long)((nx + 31) / 32) * ((ny + 13) / 14) < 3 * kSms ? 3 : 7;
+    return t;
+}
 
 static StageTune pick_tune(const fvm_handle *h, int nx, int ny) {
     const char *env = getenv("FVM_TUNE");
@@ -576,14 +594,23 @@ static GhostArgs ghost_args(fvm_handle *h, float *A, const float *B1, const floa
     return ga;
 }
 
+// A stage launch: the flat kernel on small grids, the marching one on others.
+static cudaError_t stage(fvm_handle *h, int which, int in, int blend, const StepArgs &a) {
+    const int sch = h->ext.flux_scheme, lim = h->ext.limiter, pairs = h->tune.flat_pairs;
+    if (pairs) return launch_stage_flat(which, sch, lim, pairs, h->buf[in], h->buf[blend], a, h->stream);
+    return launch_stage(which, sch, lim, h->tune, h->tm_in[in], h->tm_ctr[blend], a, h->stream);
+}
+
+// A viscous half step, with its own tile height.
+static cudaError_t viscous_pass(fvm_handle *h, int in, StepArgs a) {
+    if (h->tune.visc_rows) a.rows_per_cta = h->tune.visc_rows;
+    return launch_viscous(h->tune, h->tm_in[in], a, h->stream);
+}
+
 // One step's launches; leaves U^{n+1} in buf[BUF_X] (the caller swaps).
 static int enqueue_step(fvm_handle *h) {
-    const int sch = h->ext.flux_scheme, lim = h->ext.limiter;
-    const StageTune &tn = h->tune;
     cudaStream_t st = h->stream;
     float *Un = h->buf[BUF_N], *Us = h->buf[BUF_S], *Ux = h->buf[BUF_X], *Ud = h->buf[BUF_D];
-    const CUtensorMap &inN = h->tm_in[BUF_N], &inS = h->tm_in[BUF_S], &inD = h->tm_in[BUF_D];
-    const CUtensorMap &ctrN = h->tm_ctr[BUF_N], &ctrD = h->tm_ctr[BUF_D];
     if (!h->prm.enable_viscosity) {
         // a marching pass followed by a ghost pass lets it launch early (its
         // few CTAs then wait on the device); a marching successor is not
@@ -591,22 +618,22 @@ static int enqueue_step(fvm_handle *h) {
         // free up first
         StepArgs a1 = step_args(h, Us, 1, 0, 1.0f);
         a1.early_launch = 1;
-        CK(timed(h, 0, [&] { return launch_stage(1, sch, lim, tn, inN, ctrN, a1, st); }));
+        CK(timed(h, 0, [&] { return stage(h, 1, BUF_N, BUF_N, a1); }));
         GhostArgs g1 = ghost_args(h, Us, Un, nullptr, 0, 0);
         CK(timed(h, 4, [&] { return launch_ghost(g1, st); }));
         StepArgs a2 = step_args(h, Ux, 1, 1, 1.0f);
         a2.disp = h->disp ? h->d_disp : nullptr;
         a2.early_launch = 1;
-        CK(timed(h, 1, [&] { return launch_stage(2, sch, lim, tn, inS, ctrN, a2, st); }));
+        CK(timed(h, 1, [&] { return stage(h, 2, BUF_S, BUF_N, a2); }));
         GhostArgs g2 = ghost_args(h, Ux, Un, Us, 1, 1);
         g2.disp = h->disp ? h->d_disp : nullptr;
         CK(timed(h, 5, [&] { return launch_ghost(g2, st); }));
     } else {
         StepArgs v1 = step_args(h, Ud, 0, 0, 0.5f);
-        CK(timed(h, 2, [&] { return launch_viscous(tn, inN, v1, st); }));
+        CK(timed(h, 2, [&] { return viscous_pass(h, BUF_N, v1); }));
         StepArgs a1 = step_args(h, Us, 1, 0, 1.0f);
         a1.early_launch = 1;
-        CK(timed(h, 0, [&] { return launch_stage(1, sch, lim, tn, inD, ctrD, a1, st); }));
+        CK(timed(h, 0, [&] { return stage(h, 1, BUF_D, BUF_D, a1); }));
         GhostArgs g1 = ghost_args(h, Us, Ud, nullptr, 0, 0);
         CK(timed(h, 4, [&] { return launch_ghost(g1, st); }));
         // stage 2 blends with the diffused U^n and overwrites it in place;
@@ -614,11 +641,11 @@ static int enqueue_step(fvm_handle *h) {
         // pass this step ran 4 % slower at 1024x512 (the Euler stage 2 gains)
         StepArgs a2 = step_args(h, Ud, 0, 0, 1.0f);
         a2.pdl = 0;
-        CK(timed(h, 1, [&] { return launch_stage(2, sch, lim, tn, inS, ctrD, a2, st); }));
+        CK(timed(h, 1, [&] { return stage(h, 2, BUF_S, BUF_D, a2); }));
         StepArgs v2 = step_args(h, Ux, 1, 2, 0.5f);
         v2.disp = h->disp ? h->d_disp : nullptr;
         v2.early_launch = 1;
-        CK(timed(h, 3, [&] { return launch_viscous(tn, inD, v2, st); }));
+        CK(timed(h, 3, [&] { return viscous_pass(h, BUF_D, v2); }));
         GhostArgs g2 = ghost_args(h, Ux, Ud, nullptr, 2, 1);
         g2.disp = h->disp ? h->d_disp : nullptr;
         CK(timed(h, 5, [&] { return launch_ghost(g2, st); }));
@@ -663,6 +690,8 @@ static unsigned long long graph_key(fvm_handle *h) {
     k = k * 131 + h->tune.nt;
     k = k * 131 + h->tune.ring;
     k = k * 1031 + h->tune.rows;
+    k = k * 1031 + h->tune.visc_rows;
+    k = k * 11 + h->tune.flat_pairs;
     k = k * 1000003ULL + (unsigned long long)h->n_ghost;
     k = k * 7 + h->ext.dt_policy;
     k = k * 1000003ULL + (unsigned long long)(uintptr_t)h->stream;
@@ -1151,30 +1180,33 @@ extern "C" int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, f
     constexpr int kRows = 13;
     const int nts[2] = {128, 256}, rings[2] = {4, 6},
               rows[kRows] = {4, 8, 16, 24, 32, 40, 48, 56, 64, 80, 96, 128, 256};
-    for (int a1 = 0; a1 < 2 && rc == FVM_OK; a1++)
-        for (int a2 = 0; a2 < 2 && rc == FVM_OK; a2++)
-            for (int a3 = 0; a3 < kRows && rc == FVM_OK; a3++) {
-                StageTune cand{nts[a1], rings[a2], rows[a3]};
-                if (rows[a3] > std::max(16, h->g.ny)) continue;
-                h->tune = cand;
-                drop_graphs(h);
-                if ((rc = build_maps(h)) != FVM_OK) break;
-                fvm_sim_params w = q;
-                if ((rc = fvm_steps(h, &w, 3)) != FVM_OK) break;  // warm (captures both graph kinds)
-                cudaEventRecord(e0, h->stream);
-                if ((rc = fvm_steps(h, &w, steps)) != FVM_OK) break;
-                cudaEventRecord(e1, h->stream);
-                cudaEventSynchronize(e1);
-                float ms = 0.0f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                ms /= steps;
-                if (ms < best_ms) {
-                    best_ms = ms;
-                    best = cand;
-                }
-                // restore the state for the next candidate (buffer roles may have swapped)
-                cudaMemcpyAsync(h->buf[BUF_N], snap, bytes, cudaMemcpyDeviceToDevice, h->stream);
-            }
+    // the default shape (with the flat stage kernel on small grids), then the
+    // marching shapes
+    std::vector<StageTune> cands{heuristic_tune(h->g.nx, h->g.ny)};
+    for (int a1 = 0; a1 < 2; a1++)
+        for (int a2 = 0; a2 < 2; a2++)
+            for (int a3 = 0; a3 < kRows; a3++)
+                if (rows[a3] <= std::max(16, h->g.ny)) cands.push_back(StageTune{nts[a1], rings[a2], rows[a3]});
+    for (const StageTune &cand : cands) {
+        h->tune = cand;
+        drop_graphs(h);
+        if ((rc = build_maps(h)) != FVM_OK) break;
+        fvm_sim_params w = q;
+        if ((rc = fvm_steps(h, &w, 3)) != FVM_OK) break;  // warm (captures both graph kinds)
+        cudaEventRecord(e0, h->stream);
+        if ((rc = fvm_steps(h, &w, steps)) != FVM_OK) break;
+        cudaEventRecord(e1, h->stream);
+        cudaEventSynchronize(e1);
+        float ms = 0.0f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        ms /= steps;
+        if (ms < best_ms) {
+            best_ms = ms;
+            best = cand;
+        }
+        // restore the state for the next candidate (buffer roles may have swapped)
+        cudaMemcpyAsync(h->buf[BUF_N], snap, bytes, cudaMemcpyDeviceToDevice, h->stream);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     h->tune = (rc == FVM_OK) ? best : before;
@@ -1232,7 +1264,7 @@ extern "C" int fvm_debug_stage1(fvm_handle *h, float dt, int with_ghost, float *
     CK(cudaGetLastError());
     float *Un = h->buf[BUF_N], *Us = h->buf[BUF_S];
     StepArgs a1 = step_args(h, Us, 1, 0, 1.0f);
-    CK(launch_stage(1, h->ext.flux_scheme, h->ext.limiter, h->tune, h->tm_in[BUF_N], h->tm_ctr[BUF_N], a1, h->stream));
+    CK(stage(h, 1, BUF_N, BUF_N, a1));
     if (with_ghost && h->n_ghost > 0) {
         GhostArgs g1 = ghost_args(h, Us, Un, nullptr, 0, 0);
         CK(launch_ghost(g1, h->stream));

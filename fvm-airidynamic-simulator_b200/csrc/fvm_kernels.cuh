@@ -9,13 +9,16 @@ struct ShapeParamsHost {
     int shape;
 };
 
-// Launch configuration of the marching stage kernels (chosen per grid class
-// by the tuner): threads per CTA (= columns of primitives staged per row),
-// TMA ring depth and rows marched per CTA.
+// Launch configuration of the step kernels (chosen per grid class by a rule or
+// the tuner): threads per CTA (= columns of primitives staged per row), TMA
+// ring depth and rows marched per CTA of the marching kernels; whether the
+// stages run on the flat kernel instead.
 struct StageTune {
     int nt;          // 128 or 256
     int ring;        // TMA ring slots (prefetch distance = ring - 3)
     int rows;        // rows per CTA
+    int visc_rows = 0;   // rows per CTA of the viscous passes (0: as rows)
+    int flat_pairs = 0;  // row pairs per tile of the flat stage kernel, 3 or 7 (0: marching stages)
 };
 
 // geometry (fvm_geometry.cu)
@@ -31,6 +34,11 @@ void launch_init(const GridDesc &g, float *U, const Freestream &fs, cudaStream_t
 // 0.5*B + 0.5*(U** from U*).  Optional phase-1 BC and CFL reduction.
 cudaError_t launch_stage(int stage, int scheme, int limiter, const StageTune &tn, const CUtensorMap &tm_in,
                          const CUtensorMap &tm_blend, const StepArgs &a, cudaStream_t st);
+// The same stage with the flat kernel (one small tile per CTA, no marching):
+// the faster one on small grids.  in, blend: the input state and the RK blend
+// partner.  Bit for bit the results of launch_stage.
+cudaError_t launch_stage_flat(int stage, int scheme, int limiter, int pairs, const float *in, const float *blend,
+                              const StepArgs &a, cudaStream_t st);
 // Viscous half step out of place: out = U + dt*D(prims(U)) on interior fluid
 // cells, copy elsewhere; optional phase-1 BC and CFL reduction.
 cudaError_t launch_viscous(const StageTune &tn, const CUtensorMap &tm_in, const StepArgs &a, cudaStream_t st);

@@ -108,6 +108,72 @@ __device__ __forceinline__ bool smem_misaligned(const unsigned char *smem, DevSc
     return true;
 }
 
+// Update of the cells of column iu in rows u0 (lane .x) and u0+1 (lane .y) and
+// what follows it in a stage: wall cells keep their state, the RK blend with
+// blend(k) (stage 2), phase-1 boundary conditions, the CFL contribution, the
+// stores and a registered display field.  st0, st1: which rows are stored;
+// m: the cells' mask word; the other arguments are update_pair's.
+template <int STAGE, bool DISP, class Blend>
+__device__ __forceinline__ void update_store_pair(const StepArgs &a, const UpdateArgs &ua, uint32_t m, int iu, int u0,
+                                                  bool st0, bool st1, bool edge_x, const f2 Uc[5], const f2 dX[5],
+                                                  const f2 dY[5], f2 du, f2 dv, f2 p_c, Blend blend,
+                                                  float &lmax_speed, unsigned &nbad) {
+    const GridDesc &g = a.g;
+    const bool ey0 = (u0 == 0 || u0 == g.ny - 1), ey1 = (u0 + 1 == 0 || u0 + 1 == g.ny - 1);
+    f2 Un[5];
+    update_pair(Uc, dX, dY, du, dv, p_c, edge_x, ey0, ey1, ua, Un);
+    // wall cells keep their state
+    if ((m & (MB_WALL * 0x0101u)) != 0u) {
+        const bool w0 = (m & MB_WALL) != 0u, w1 = (m & (MB_WALL << 8)) != 0u;
+#pragma unroll
+        for (int k = 0; k < 5; k++) Un[k] = p_sel(w0, w1, Uc[k], Un[k]);
+    }
+    if (STAGE == 2) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) Un[k] = p_fma(splat(0.5f), Un[k], p_mul(splat(0.5f), blend(k)));
+    }
+    // phase-1 conditions act only on non-fluid cells and the domain's edge cells
+    const uint32_t ct0 = mb_type(m), ct1 = mb_type(m >> 8);
+    if (a.apply_bc && ((m & kTypeBits) != 0u || edge_x || ey0 || ey1)) {
+        float Ur[2][5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            Ur[0][k] = Un[k].x;
+            Ur[1][k] = Un[k].y;
+        }
+        if (st0) bc_pointwise(Ur[0], ct0, iu, u0, g.nx, g.ny, a.fs);
+        if (st1) bc_pointwise(Ur[1], ct1, iu, u0 + 1, g.nx, g.ny, a.fs);
+#pragma unroll
+        for (int k = 0; k < 5; k++) Un[k] = mk2(Ur[0][k], Ur[1][k]);
+    }
+    if (a.cfl) {
+        const f2 ws = pair_wave_speed(Un);
+        const bool c0 = st0 && ct0 != CT_GHOST, c1 = st1 && ct1 != CT_GHOST;
+        lmax_speed = fmaxf(lmax_speed, fmaxf(c0 ? ws.x : 0.0f, c1 ? ws.y : 0.0f));
+        nbad += pair_nonfinite(Un, c0, c1);
+    }
+    float *dst = a.out + iu + (size_t)u0 * g.pitch;
+    if (st0) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) dst[k * g.plane] = Un[k].x;
+    }
+    if (st1) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) dst[k * g.plane + g.pitch] = Un[k].y;
+    }
+    // a registered display field of the step's result (the descriptor is read
+    // here, not held in registers)
+    if (DISP && STAGE == 2) {
+        float *const dptr = a.disp->ptr;
+        if (dptr) {
+            const int kind = a.disp->kind;
+            float *d = dptr + (size_t)u0 * g.nx + iu;
+            if (st0) d[0] = derived_value(kind, Un[0].x, Un[1].x, Un[2].x, Un[4].x);
+            if (st1) d[g.nx] = derived_value(kind, Un[0].y, Un[1].y, Un[2].y, Un[4].y);
+        }
+    }
+}
+
 template <int NT, int K, int STAGE>
 struct StageLayout {
     static constexpr int W = NT - 4;   // output columns
@@ -258,7 +324,6 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
     const bool edge_x = (iu == 0 || iu == nx - 1);
     const int tx = min(t, W);
     const int cy = min(t, W - 1) + 2;
-    float *outp = a.out + iu;
 
     int kr = base % KP, par = (base / KP) & 1, ku = (base + KP - 1) % KP;
     int s0 = 0, s1 = 1;  // primitive / mask ring slots of row pairs q, q-1
@@ -325,7 +390,7 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
             const bool st0 = col_ok && u0 >= j0 && u0 < j1, st1 = col_ok && u0 + 1 >= j0 && u0 + 1 < j1;
             if (st0 || st1) {
                 const float *src = raw + (size_t)(ku * 2) * L::SLOT;
-                f2 Uc[5], Un[5];
+                f2 Uc[5];
 #pragma unroll
                 for (int k = 0; k < 5; k++)
                     Uc[k] = mk2(ring_at<L::NB>(src, k, t + 4), ring_at<L::NB>(src + L::SLOT, k, t + 4));
@@ -340,60 +405,9 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
 #pragma unroll
                 for (int k = 0; k < 5; k++) dY[k] = mk2(Fy[k].x - fyB[k], Fy[k].y - Fy[k].x);
                 const f2 dv = mk2(vfy.x - vfB, vfy.y - vfy.x);
-                const bool ey0 = (u0 == 0 || u0 == ny - 1), ey1 = (u0 + 1 == 0 || u0 + 1 == ny - 1);
-                update_pair(Uc, dX, dY, du, dv, mk2(B1.z, B1.w), edge_x, ey0, ey1, ua, Un);
-                // wall cells keep their state
-                if ((my & (MB_WALL * 0x0101u)) != 0u) {
-                    const bool w0 = (my & MB_WALL) != 0u, w1 = (my & (MB_WALL << 8)) != 0u;
-#pragma unroll
-                    for (int k = 0; k < 5; k++) Un[k] = p_sel(w0, w1, Uc[k], Un[k]);
-                }
-                if (STAGE == 2) {
-                    const float *b = bl + t;
-#pragma unroll
-                    for (int k = 0; k < 5; k++)
-                        Un[k] = p_fma(splat(0.5f), Un[k], p_mul(splat(0.5f), mk2(b[k * W], b[L::BSLOT + k * W])));
-                }
-// phase-1 conditions act only on non-fluid cells and the domain's edge cells
-                const uint32_t ct0 = mb_type(my), ct1 = mb_type(my >> 8);
-                if (a.apply_bc && ((my & kTypeBits) != 0u || edge_x || ey0 || ey1)) {
-                    float Ur[2][5];
-#pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        Ur[0][k] = Un[k].x;
-                        Ur[1][k] = Un[k].y;
-                    }
-                    if (st0) bc_pointwise(Ur[0], ct0, iu, u0, nx, ny, a.fs);
-                    if (st1) bc_pointwise(Ur[1], ct1, iu, u0 + 1, nx, ny, a.fs);
-#pragma unroll
-                    for (int k = 0; k < 5; k++) Un[k] = mk2(Ur[0][k], Ur[1][k]);
-                }
-                if (a.cfl) {
-                    const f2 ws = pair_wave_speed(Un);
-                    const bool c0 = st0 && ct0 != CT_GHOST, c1 = st1 && ct1 != CT_GHOST;
-                    lmax_speed = fmaxf(lmax_speed, fmaxf(c0 ? ws.x : 0.0f, c1 ? ws.y : 0.0f));
-                    nbad += pair_nonfinite(Un, c0, c1);
-                }
-                float *dst = outp + (size_t)u0 * g.pitch;
-                if (st0) {
-#pragma unroll
-                    for (int k = 0; k < 5; k++) dst[k * g.plane] = Un[k].x;
-                }
-                if (st1) {
-#pragma unroll
-                    for (int k = 0; k < 5; k++) dst[k * g.plane + g.pitch] = Un[k].y;
-                }
-                // a registered display field of the step's result (the descriptor
-                // is read here, not held in registers across the loop)
-                if (DISP && STAGE == 2) {
-                    float *const dptr = a.disp->ptr;
-                    if (dptr) {
-                        const int kind = a.disp->kind;
-                        float *d = dptr + (size_t)u0 * nx + iu;
-                        if (st0) d[0] = derived_value(kind, Un[0].x, Un[1].x, Un[2].x, Un[4].x);
-                        if (st1) d[nx] = derived_value(kind, Un[0].y, Un[1].y, Un[2].y, Un[4].y);
-                    }
-                }
+                update_store_pair<STAGE, DISP>(
+                    a, ua, my, iu, u0, st0, st1, edge_x, Uc, dX, dY, du, dv, mk2(B1.z, B1.w),
+                    [&](int k) { return mk2(bl[k * W + t], bl[L::BSLOT + k * W + t]); }, lmax_speed, nbad);
             }
         }
 #pragma unroll
@@ -499,6 +513,135 @@ __global__ void __launch_bounds__(NT, 768 / NT)
     if (a.early_launch) pdl_trigger();
     if (!ok) return;
     if (a.cfl) block_publish<NT>(lmax, 0.0f, nbad, a.sc);
+}
+
+// ---- flat stage kernel: one tile of 32 columns x 2 PAIRS rows per CTA, with a
+// thread for every face pair of the tile at once instead of a march over row
+// pairs.
+//   1. primitives and mask words of the tile and its two-cell halo from global
+//      memory into shared memory
+//   -- barrier --
+//   2. thread (face f, pair p): the x-faces left of column i0+f in rows 2p,
+//      2p+1 of the tile, to shared memory; then thread (column c, pair p),
+//      p = -1 .. PAIRS-1: the y-faces (2p | 2p+1), (2p+1 | 2p+2), kept in
+//      registers, the upper one also to shared memory for the pair above
+//   -- barrier --
+//   3. update of rows 2p, 2p+1 at column c; the cells' state comes from global
+//      memory again (L1 hits of step 1)
+// For small grids: bound by the latency of one tile's dependent arithmetic
+// (two Riemann solves, one update) and the launches, not by issue slots.
+// 64 registers, 32 warps per SM: at 80 registers and 24 warps 1501x777 took
+// 78.0 us a step instead of 73.0, at 16 warps 90.  The arithmetic is that of
+// the marching kernel, function for function, so both give the same bits.
+template <int PAIRS>
+struct FlatTile {
+    static constexpr int X = 32, ROWS = 2 * PAIRS;
+    static constexpr int THREADS = X * (PAIRS + 1);
+    static constexpr int COLS = X + 4, SLOTS = PAIRS + 2;
+    static_assert(THREADS >= PAIRS * (X + 1), "one x-face pair per thread");
+};
+
+template <int PAIRS, int STAGE, int SCHEME, int LIM, bool DISP>
+__global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIRS>::THREADS)
+    k_stage_flat(const StepArgs a, const float *in, const float *blend) {
+    using L = FlatTile<PAIRS>;
+    __shared__ float4 PA[L::SLOTS][L::COLS], PB[L::SLOTS][L::COLS];
+    __shared__ float4 XA[PAIRS][L::X + 1], XB[PAIRS][L::X + 1], XC[PAIRS][L::X + 1];
+    __shared__ float YU[6][PAIRS][L::X];  // upper y-face of pair p-1: fluxes and face velocity
+    __shared__ uint16_t M[L::SLOTS][L::COLS];
+    const GridDesc &g = a.g;
+    const int nx = g.nx, ny = g.ny;
+    const int t = threadIdx.x;
+    const int i0 = blockIdx.x * L::X, j0 = blockIdx.y * L::ROWS;
+    pdl_wait();
+    const UpdateArgs ua{a.sc->dt * a.dt_scale, 1.0f / g.dx, 1.0f / g.dy};
+    for (int k = t; k < L::SLOTS * L::COLS; k += L::THREADS) {
+        const int s = k / L::COLS, x = k - s * L::COLS;
+        const int col = clampi(i0 - 2 + x, 0, nx - 1);
+        float rho[2], u[2], v[2], p[2], T;
+        uint32_t m = 0u;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const size_t c = (size_t)clampi(j0 - 2 + 2 * s + h, 0, ny - 1) * g.pitch + col;
+            const float *U = in + c;
+            rho[h] = __ldg(U);
+            prim_from_cons(rho[h], __ldg(U + g.plane), __ldg(U + 2 * g.plane), __ldg(U + 3 * g.plane),
+                           __ldg(U + 4 * g.plane), u[h], v[h], p[h], T);
+            m |= (uint32_t)__ldg(a.mask + c) << (8 * h);
+        }
+        M[s][x] = (uint16_t)m;
+        PA[s][x] = make_float4(rho[0], rho[1], u[0], u[1]);
+        PB[s][x] = make_float4(v[0], v[1], p[0], p[1]);
+    }
+    __syncthreads();
+    // the blend partner's rows (128 bytes each), needed two phases later
+    if (STAGE == 2 && t < 5 * L::ROWS && j0 + t / 5 < ny)
+        prefetch_l2(blend + (size_t)(t % 5) * g.plane + (size_t)(j0 + t / 5) * g.pitch + i0);
+    // x-faces
+    if (t < PAIRS * (L::X + 1)) {
+        const int p = t / (L::X + 1), f = t - p * (L::X + 1);
+        const float4 *A = &PA[p + 1][f], *B = &PB[p + 1][f];
+        const PairPrim c0 = pair_prim(A[0], B[0]), c1 = pair_prim(A[1], B[1]), c2 = pair_prim(A[2], B[2]),
+                       c3 = pair_prim(A[3], B[3]);
+        const PairSl sa{p_half_slope<LIM>(c0.rho, c1.rho, c2.rho), p_half_slope<LIM>(c0.u, c1.u, c2.u),
+                        p_half_slope<LIM>(c0.v, c1.v, c2.v), p_half_slope<LIM>(c0.p, c1.p, c2.p)};
+        const PairSl sb{p_half_slope<LIM>(c1.rho, c2.rho, c3.rho), p_half_slope<LIM>(c1.u, c2.u, c3.u),
+                        p_half_slope<LIM>(c1.v, c2.v, c3.v), p_half_slope<LIM>(c1.p, c2.p, c3.p)};
+        f2 F[5];
+        face_pair_core<true, SCHEME>(M[p + 1][f + 1], c1, sa, c2, sb, F);
+        const f2 vel = p_face_velocity(F[0], c1.rho, c2.rho);
+        XA[p][f] = make_float4(F[0].x, F[0].y, F[1].x, F[1].y);
+        XB[p][f] = make_float4(F[2].x, F[2].y, F[3].x, F[3].y);
+        XC[p][f] = make_float4(F[4].x, F[4].y, vel.x, vel.y);
+    }
+    // y-faces; pair -1 only for its upper face
+    const int c = t & (L::X - 1), p = (t / L::X) - 1;
+    f2 Fy[5];
+    f2 vfy;
+    {
+        const int x = c + 2;
+        const float4 Al = PA[max(p, 0)][x], Bl = PB[max(p, 0)][x];
+        const PairPrim lo = pair_prim(PA[p + 1][x], PB[p + 1][x]), hi = pair_prim(PA[p + 2][x], PB[p + 2][x]);
+        const PairPrim mid{mk2(lo.rho.y, hi.rho.x), mk2(lo.u.y, hi.u.x), mk2(lo.v.y, hi.v.x), mk2(lo.p.y, hi.p.x)};
+        // half slopes of row 2p, {rho, u} and {v, p} as lanes
+        const f2 sru = p_half_slope<LIM>(mk2(Al.y, Al.w), mk2(lo.rho.x, lo.u.x), mk2(lo.rho.y, lo.u.y));
+        const f2 svp = p_half_slope<LIM>(mk2(Bl.y, Bl.w), mk2(lo.v.x, lo.p.x), mk2(lo.v.y, lo.p.y));
+        float sy[4] = {sru.x, svp.x, sru.y, svp.y};
+        face_pair_y<SCHEME, LIM>(M[p + 1][x], lo, mid, hi, sy, Fy);
+        vfy = p_face_velocity(Fy[0], lo.rho, mid.rho);
+    }
+    if (p < PAIRS - 1) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) YU[k][p + 1][c] = Fy[k].y;
+        YU[5][p + 1][c] = vfy.y;
+    }
+    __syncthreads();
+    float lmax = 0.0f;
+    unsigned nbad = 0;
+    const int iu = i0 + c, u0 = j0 + 2 * p;
+    if (p >= 0 && iu < nx && u0 < ny) {
+        const bool st1 = u0 + 1 < ny;
+        const size_t cell = (size_t)u0 * g.pitch + iu, up = st1 ? cell + g.pitch : cell;
+        f2 Uc[5], dY[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            Uc[k] = mk2(__ldg(in + k * g.plane + cell), __ldg(in + k * g.plane + up));
+            dY[k] = mk2(Fy[k].x - YU[k][p][c], Fy[k].y - Fy[k].x);
+        }
+        const float4 LA = XA[p][c], RA = XA[p][c + 1], LB = XB[p][c], RB = XB[p][c + 1], LC = XC[p][c],
+                     RC = XC[p][c + 1];
+        const f2 dX[5] = {p_sub(mk2(RA.x, RA.y), mk2(LA.x, LA.y)), p_sub(mk2(RA.z, RA.w), mk2(LA.z, LA.w)),
+                          p_sub(mk2(RB.x, RB.y), mk2(LB.x, LB.y)), p_sub(mk2(RB.z, RB.w), mk2(LB.z, LB.w)),
+                          p_sub(mk2(RC.x, RC.y), mk2(LC.x, LC.y))};
+        const f2 du = p_sub(mk2(RC.z, RC.w), mk2(LC.z, LC.w));
+        const f2 dv = mk2(vfy.x - YU[5][p][c], vfy.y - vfy.x);
+        const float4 B1 = PB[p + 1][c + 2];
+        update_store_pair<STAGE, DISP>(
+            a, ua, M[p + 1][c + 2], iu, u0, true, st1, iu == 0 || iu == nx - 1, Uc, dX, dY, du, dv, mk2(B1.z, B1.w),
+            [&](int k) { return mk2(blend[k * g.plane + cell], blend[k * g.plane + up]); }, lmax, nbad);
+    }
+    if (a.early_launch) pdl_trigger();
+    if (a.cfl) block_publish<L::THREADS>(lmax, 0.0f, nbad, a.sc);
 }
 
 template <int NT, int K>
@@ -1281,6 +1424,33 @@ static cudaError_t launch_stage_s(int scheme, int lim, const StageTune &tn, cons
     if (scheme == 0 && lim == 1) return launch_stage_t<NT, K, STAGE, 0, 1>(tn, tm_in, tm_blend, a, st);
     if (scheme == 1 && lim == 0) return launch_stage_t<NT, K, STAGE, 1, 0>(tn, tm_in, tm_blend, a, st);
     return launch_stage_t<NT, K, STAGE, 1, 1>(tn, tm_in, tm_blend, a, st);
+}
+
+template <int PAIRS, int STAGE, int SCHEME, int LIM>
+static cudaError_t launch_flat_t(const float *in, const float *blend, const StepArgs &a, cudaStream_t st) {
+    using L = FlatTile<PAIRS>;
+    auto kern = (STAGE == 2 && a.disp) ? k_stage_flat<PAIRS, STAGE, SCHEME, LIM, STAGE == 2>
+                                       : k_stage_flat<PAIRS, STAGE, SCHEME, LIM, false>;
+    dim3 grid((a.g.nx + L::X - 1) / L::X, (a.g.ny + L::ROWS - 1) / L::ROWS);
+    return launch_step_kernel(a.pdl != 0, kern, grid, dim3(L::THREADS), 0, st, a, in, blend);
+}
+
+template <int PAIRS, int STAGE>
+static cudaError_t launch_flat_s(int scheme, int lim, const float *in, const float *blend, const StepArgs &a,
+                                 cudaStream_t st) {
+    if (scheme == 0 && lim == 0) return launch_flat_t<PAIRS, STAGE, 0, 0>(in, blend, a, st);
+    if (scheme == 0 && lim == 1) return launch_flat_t<PAIRS, STAGE, 0, 1>(in, blend, a, st);
+    if (scheme == 1 && lim == 0) return launch_flat_t<PAIRS, STAGE, 1, 0>(in, blend, a, st);
+    return launch_flat_t<PAIRS, STAGE, 1, 1>(in, blend, a, st);
+}
+
+cudaError_t launch_stage_flat(int stage, int scheme, int limiter, int pairs, const float *in, const float *blend,
+                              const StepArgs &a, cudaStream_t st) {
+    if (pairs == 3)
+        return stage == 1 ? launch_flat_s<3, 1>(scheme, limiter, in, blend, a, st)
+                          : launch_flat_s<3, 2>(scheme, limiter, in, blend, a, st);
+    return stage == 1 ? launch_flat_s<7, 1>(scheme, limiter, in, blend, a, st)
+                      : launch_flat_s<7, 2>(scheme, limiter, in, blend, a, st);
 }
 
 cudaError_t launch_stage(int stage, int scheme, int limiter, const StageTune &tn, const CUtensorMap &tm_in,

@@ -98,6 +98,9 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Fetch the line at p into L2.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Warp max of a non-negative float (NaN-free inputs assumed by the callers).
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll

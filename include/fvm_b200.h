@@ -259,17 +259,18 @@ typedef struct fvm_kernel_time {
 int fvm_set_kernel_timing(fvm_handle *h, int enable);
 int fvm_kernel_times(fvm_handle *h, fvm_kernel_time *out, int cap, int *count_out);
 
-/* Autotuner: times every candidate launch tuning of the marching step
- * kernels (threads per CTA 128/256, TMA ring depth 4/6 rows, rows per CTA
- * 4..256) over `steps` steps of this solve, restoring the state after each,
+/* Autotuner: times the default launch shape (on small grids: stages on the
+ * flat kernel) and every candidate launch tuning of the marching step kernels
+ * (threads per CTA 128/256, TMA ring depth 4/6 rows, rows per CTA 4..256) over `steps` steps of this solve, restoring the state after each,
  * keeps the fastest for this handle and caches it for the grid class (grid
  * size, viscous flag, flux scheme, limiter) for later handles in the process.
  * *best_ms_out receives the winner's time per step. */
 int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, float *best_ms_out);
-/* The launch tuning in use. */
+/* The launch tuning of the marching kernels in use (by default small grids run
+ * their stages on the flat kernel, which this tuning does not describe). */
 int fvm_get_tune(fvm_handle *h, int *nt, int *ring, int *rows);
-/* Pin a launch tuning (e.g. one an earlier fvm_autotune chose): threads per
- * CTA 128 or 256, ring depth 4 or 6 rows, an even number of rows per CTA in
+/* Pin a launch tuning (e.g. one an earlier fvm_autotune chose) of the marching
+ * kernels, which then run on every grid size: threads per CTA 128 or 256, ring depth 4 or 6 rows, an even number of rows per CTA in
  * 4..65536.  Results are bitwise the same under every allowed tuning; only the
  * speed differs.  (Tiles start on even rows, so a row always takes the same
  * place in the row pair the kernels evaluate together; the two places are
