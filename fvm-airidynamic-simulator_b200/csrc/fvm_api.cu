@@ -194,6 +194,7 @@ static cudaError_t timed(fvm_handle *h, int kernel, F fn) {
 }
 
 static void drop_graphs(fvm_handle *h) {
+    h->plain_steps = 0;
     for (int k = 0; k < 2; k++) {
         if (h->graph[k]) cudaGraphExecDestroy(h->graph[k]);
         h->graph[k] = nullptr;
@@ -741,6 +742,28 @@ static int state_parity(fvm_handle *h) {
     return (h->buf[BUF_N] == h->parity_base) ? 0 : 1;
 }
 
+// Steps after which the step graphs are captured.  Capturing and instantiating
+// both parities costs 0.2 ms on the host; a step's four to six plain launches
+// cost it 10-15 us, hidden behind the 16 us and more of the kernels, so a graph
+// saves at most 4 us a step (NS 1024x512: 59.6 against 63.3 us; Euler steps are
+// the same either way).  A solve whose geometry or parameters change every few
+// steps therefore never captures; a call long enough to earn the capture back
+// does at once.
+constexpr int kGraphAfter = 16, kGraphLongCall = 64;
+
+// Whether the next n steps run as graphs: the one they need exists, or enough
+// steps have run (or very many are asked for) to capture it.  A stream that is itself
+// being captured keeps to the graphs.
+static bool want_graphs(fvm_handle *h, int n) {
+    if (h->plain_steps >= kGraphAfter || n > kGraphLongCall) return true;
+    const unsigned long long key = graph_key(h);
+    const int par = state_parity(h);
+    if (n >= 2 && h->graph[par] && h->graph_key[par] == key) return true;
+    if (n == 1 && h->graph1[par] && h->graph1_key[par] == key) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(h->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+}
+
 // Captured graphs of `nsteps` steps (2 or 1) for both buffer parities, built
 // together the first time either is needed (and again after a change of
 // their key), so no later call pays for a capture and an instantiation.  The
@@ -809,7 +832,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     }
     if (int r = prepare_dt(h, p)) return r;
     const bool use_graph = !h->timing && h->stream != nullptr && h->stream != cudaStreamLegacy &&
-                           h->stream != cudaStreamPerThread && getenv("FVM_NO_GRAPH") == nullptr;
+                           h->stream != cudaStreamPerThread && getenv("FVM_NO_GRAPH") == nullptr && want_graphs(h, n);
     int done = 0;
     if (use_graph && n >= 2) {
         const int par = state_parity(h);
@@ -832,6 +855,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     for (; done < n; done++) {
         if (int r = enqueue_step(h)) return r;
         swap_state(h);
+        h->plain_steps++;
     }
     const int rf = finish_steps(h, p, n);
     h->disp_fresh = rf == FVM_OK && h->disp != nullptr;

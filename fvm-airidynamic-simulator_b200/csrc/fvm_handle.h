@@ -54,6 +54,7 @@ struct fvm_handle {
     // graph replay of one step (single-step calls and odd remainders), per parity
     cudaGraphExec_t graph1[2] = {nullptr, nullptr};
     unsigned long long graph1_key[2] = {0, 0};
+    int plain_steps = 0;         // steps launched plainly since the graphs were dropped
     // registered display field (fvm_set_display_field): the last passes of
     // every step write it (destination and kind in the device descriptor
     // d_disp, mirrored in disp / disp_kind); fresh while the state is the one
