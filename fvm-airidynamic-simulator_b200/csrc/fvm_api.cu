@@ -359,21 +359,27 @@ static int build_geometry(fvm_handle *h, bool fixup) {
     CK(cudaGetLastError());
     launch_mask(h->g, h->ct, h->mask, h->stream);
     CK(cudaGetLastError());
-    CK(cudaMemsetAsync(h->d_count, 0, sizeof(int), h->stream));
-    launch_ghost_table(h->g, h->sdf, h->ct, nullptr, 0, h->d_count, h->stream);
-    CK(cudaGetLastError());
-    int n = 0;
-    CK(cudaMemcpyAsync(&n, h->d_count, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    // one pass fills the table and counts; only a table that proves too small
+    // (the first one) is allocated and filled again
+    int *const count = reinterpret_cast<int *>(h->h_res);
+    auto fill = [&]() -> int {
+        CK(cudaMemsetAsync(h->d_count, 0, sizeof(int), h->stream));
+        launch_ghost_table(h->g, h->sdf, h->ct, h->ghosts, h->ghost_cap, h->d_count, h->stream);
+        CK(cudaGetLastError());
+        return FVM_OK;
+    };
+    if (int r = fill()) return r;
+    CK(cudaMemcpyAsync(count, h->d_count, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    const int n = *count;
     if (n > h->ghost_cap) {
         if (h->ghosts) cudaFree(h->ghosts);
         h->ghosts = nullptr;
+        h->ghost_cap = h->n_ghost = 0;
+        CKA(cudaMalloc(&h->ghosts, (size_t)std::max(n, 64) * sizeof(GhostInfo)));
         h->ghost_cap = std::max(n, 64);
-        CKA(cudaMalloc(&h->ghosts, (size_t)h->ghost_cap * sizeof(GhostInfo)));
+        if (int r = fill()) return r;
     }
-    CK(cudaMemsetAsync(h->d_count, 0, sizeof(int), h->stream));
-    if (n > 0) launch_ghost_table(h->g, h->sdf, h->ct, h->ghosts, h->ghost_cap, h->d_count, h->stream);
-    CK(cudaGetLastError());
     h->n_ghost = n;
     drop_graphs(h);
     return FVM_OK;
@@ -381,10 +387,8 @@ static int build_geometry(fvm_handle *h, bool fixup) {
 
 // Boundary conditions on the current state (both phases), set-up path.
 static int apply_bc_full(fvm_handle *h) {
-    CK(launch_bc_phase1(h->g, h->Un, h->mask, freestream(h->prm), h->stream));
+    CK(launch_bc_phase1(h->g, h->Un, h->mask, freestream(h->prm), h->buf[BUF_S], h->stream));
     if (h->n_ghost > 0) {
-        CK(cudaMemcpyAsync(h->buf[BUF_S], h->Un, (size_t)h->g.plane * 5 * sizeof(float), cudaMemcpyDeviceToDevice,
-                           h->stream));
         GhostArgs ga{};
         ga.g = h->g;
         ga.list = h->ghosts;
@@ -426,12 +430,13 @@ extern "C" int fvm_create(fvm_handle **out) {
     if (cudaMalloc(&h->sc, sizeof(DevScalars)) != cudaSuccess || cudaMalloc(&h->d_count, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&h->d_tmp, 16) != cudaSuccess || cudaMalloc(&h->d_counter, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&h->d_disp, sizeof(DisplayDesc)) != cudaSuccess ||
-        cudaMallocHost(&h->h_sc, sizeof(DevScalars) + 8 * sizeof(double)) != cudaSuccess) {
+        cudaMallocHost(&h->h_sc, sizeof(DevScalars) + 8 * sizeof(double) + sizeof(HostScalars)) != cudaSuccess) {
         delete h;
         return set_err(FVM_ERR_ALLOC, "fvm_create: allocation failed");
     }
     static_assert(sizeof(DevScalars) % alignof(double) == 0, "the results follow the mirror");
     h->h_res = reinterpret_cast<double *>(h->h_sc + 1);
+    h->h_now = reinterpret_cast<HostScalars *>(h->h_res + 8);
     cudaMemsetAsync(h->sc, 0, sizeof(DevScalars), h->stream);
     cudaMemsetAsync(h->d_disp, 0, sizeof(DisplayDesc), h->stream);
     cudaMemsetAsync(h->d_tmp, 0, 16, h->stream);
@@ -491,6 +496,7 @@ extern "C" int fvm_reset(fvm_handle *h, const fvm_sim_params *p) {
     h->g.dx = p->dx;
     h->g.dy = p->dy;
     k_zero_scalars<<<1, 1, 0, h->stream>>>(h->sc);
+    h->now_valid = false;
     h->launches_at_sc_copy = -1;  // the host copy of the scalars is out of date
     CK(cudaGetLastError());
     launch_init(h->g, h->Un, freestream(h->prm), h->stream);
@@ -608,8 +614,12 @@ static cudaError_t viscous_pass(fvm_handle *h, int in, StepArgs a) {
     return launch_viscous(h->tune, h->tm_in[in], a, h->stream);
 }
 
-// One step's launches; leaves U^{n+1} in buf[BUF_X] (the caller swaps).
-static int enqueue_step(fvm_handle *h) {
+// One step's launches; leaves U^{n+1} in buf[BUF_X] (the caller swaps).  to_host:
+// its last pass writes the scalars to the host as well.  Only the last step of
+// a call does: completing the writes across the bus holds the next step back
+// (256x128: 17.4 us a step instead of 16.4 when every step did), but spares
+// the host a copy (one step, its time step and back: 43 -> 34 us).
+static int enqueue_step(fvm_handle *h, bool to_host) {
     cudaStream_t st = h->stream;
     float *Un = h->buf[BUF_N], *Us = h->buf[BUF_S], *Ux = h->buf[BUF_X], *Ud = h->buf[BUF_D];
     if (!h->prm.enable_viscosity) {
@@ -627,6 +637,7 @@ static int enqueue_step(fvm_handle *h) {
         a2.early_launch = 1;
         CK(timed(h, 1, [&] { return stage(h, 2, BUF_S, BUF_N, a2); }));
         GhostArgs g2 = ghost_args(h, Ux, Un, Us, 1, 1);
+        g2.host = to_host ? h->h_now : nullptr;
         g2.disp = h->disp ? h->d_disp : nullptr;
         CK(timed(h, 5, [&] { return launch_ghost(g2, st); }));
     } else {
@@ -648,6 +659,7 @@ static int enqueue_step(fvm_handle *h) {
         v2.early_launch = 1;
         CK(timed(h, 3, [&] { return viscous_pass(h, BUF_D, v2); }));
         GhostArgs g2 = ghost_args(h, Ux, Ud, nullptr, 2, 1);
+        g2.host = to_host ? h->h_now : nullptr;
         g2.disp = h->disp ? h->d_disp : nullptr;
         CK(timed(h, 5, [&] { return launch_ghost(g2, st); }));
     }
@@ -705,30 +717,43 @@ static unsigned long long graph_key(fvm_handle *h) {
     return k;
 }
 
-// Status of the error word in the host copy of the device scalars.
-static int device_error_status(fvm_handle *h) {
-    if (h->h_sc->err & kErrTimeout)
-        return set_err(FVM_ERR_TIMEOUT, "a bounded device wait expired (error word 0x%x)", h->h_sc->err);
-    if (h->h_sc->err & kErrSmemAlign)
+// Status of a device error word.
+static int error_status(unsigned err) {
+    if (err & kErrTimeout) return set_err(FVM_ERR_TIMEOUT, "a bounded device wait expired (error word 0x%x)", err);
+    if (err & kErrSmemAlign)
         return set_err(FVM_ERR_CUDA, "shared-memory staging area not 128-byte aligned; step skipped (error word 0x%x)",
-                       h->h_sc->err);
+                       err);
+    return FVM_OK;
+}
+
+// The scalars on the host, once the stream is idle: as the last kernel that
+// changed them wrote them, or else copied.
+static int sync_scalars(fvm_handle *h) {
+    if (h->now_valid) {
+        CK(cudaStreamSynchronize(h->stream));
+        return FVM_OK;
+    }
+    CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    const DevScalars &d = *h->h_sc;
+    *h->h_now = HostScalars{{d.cfl[0], d.cfl[1]}, d.dt_last, d.t, d.err, 0u};
     return FVM_OK;
 }
 
 static int check_device_error(fvm_handle *h) {
-    CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    return device_error_status(h);
+    if (int r = sync_scalars(h)) return r;
+    return error_status(h->h_now->err);
 }
 
-static int finish_steps(fvm_handle *h, fvm_sim_params *p, int n) {
+static int finish_steps(fvm_handle *h, fvm_sim_params *p, int n, bool to_host) {
+    h->now_valid = to_host;
     if (h->ext.dt_policy == FVM_DT_FIXED) {
         for (int k = 0; k < n; k++) p->t_current += p->dt;
         p->step += n;
     } else {
         if (int r = check_device_error(h)) return r;
-        p->dt = h->h_sc->dt_last;
-        p->t_current = h->h_sc->t;
+        p->dt = h->h_now->dt_last;
+        p->t_current = h->h_now->t;
         p->step += n;
     }
     h->cfl_valid = true;
@@ -789,10 +814,11 @@ static int ensure_graphs(fvm_handle *h, int nsteps, cudaGraphExec_t *graphs, uns
         long long before = h->launches;
         // two steps swap the state twice (also when a step fails to enqueue),
         // one step not at all: the pointers end as they began
-        int r = enqueue_step(h);
+        // (the one-step graph is always a call's last step)
+        int r = enqueue_step(h, nsteps == 1);
         if (nsteps == 2) {
             swap_state(h);
-            if (!r) r = enqueue_step(h);
+            if (!r) r = enqueue_step(h, false);
             swap_state(h);
         }
         cudaError_t ec = cudaStreamEndCapture(h->stream, &gr);
@@ -819,6 +845,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     if (n < 0) return set_err(FVM_ERR_INVALID, "negative step count");
     if (n == 0) return FVM_OK;
     h->disp_fresh = false;  // until every step is queued
+    h->now_valid = false;
     // per-step knobs the reference reads from params on every call
     h->prm.cfl = p->cfl;
     h->prm.cfl_visc = p->cfl_visc;
@@ -834,6 +861,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     const bool use_graph = !h->timing && h->stream != nullptr && h->stream != cudaStreamLegacy &&
                            h->stream != cudaStreamPerThread && getenv("FVM_NO_GRAPH") == nullptr && want_graphs(h, n);
     int done = 0;
+    bool to_host = false;  // whether the last step queued writes the scalars to the host
     if (use_graph && n >= 2) {
         const int par = state_parity(h);
         if (int r = ensure_graphs(h, 2, h->graph, h->graph_key)) return r;
@@ -850,14 +878,16 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
         CK(cudaGraphLaunch(h->graph1[par], h->stream));
         h->launches += h->prm.enable_viscosity ? 6 : 4;
         swap_state(h);
+        to_host = true;
         done++;
     }
     for (; done < n; done++) {
-        if (int r = enqueue_step(h)) return r;
+        to_host = done == n - 1;
+        if (int r = enqueue_step(h, to_host)) return r;
         swap_state(h);
         h->plain_steps++;
     }
-    const int rf = finish_steps(h, p, n);
+    const int rf = finish_steps(h, p, n, to_host);
     h->disp_fresh = rf == FVM_OK && h->disp != nullptr;
     return rf;
 }
@@ -869,8 +899,16 @@ extern "C" int fvm_synchronize(fvm_handle *h) {
     // only kernels set the error word: when none was launched since
     // fvm_queue_dt copied the device scalars (the reference's per-frame
     // queue / synchronize / read sequence), that copy, complete now, holds it
-    if (h->launches == h->launches_at_sc_copy) return device_error_status(h);
+    if (h->launches == h->launches_at_sc_copy) return error_status(h->h_sc->err);
     return check_device_error(h);
+}
+
+static int queue_cfl(fvm_handle *h) {
+    CK(launch_cfl_state(h->g, h->Un, h->mask, h->sc, h->h_now, h->stream));
+    h->launches++;
+    h->cfl_valid = true;
+    h->now_valid = true;
+    return FVM_OK;
 }
 
 // CFL maxima of the current state: after a step they come from the fused
@@ -878,14 +916,11 @@ extern "C" int fvm_synchronize(fvm_handle *h) {
 // otherwise from a standalone pass over the state.
 static int cfl_maxima(fvm_handle *h, float *ms, float *mn) {
     if (!h->cfl_valid) {
-        CK(launch_cfl_state(h->g, h->Un, h->mask, h->sc, h->stream));
-        h->launches++;
-        h->cfl_valid = true;
+        if (int r = queue_cfl(h)) return r;
     }
-    CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    *ms = h->h_sc->cfl[0];
-    *mn = h->h_sc->cfl[1];
+    if (int r = sync_scalars(h)) return r;
+    *ms = h->h_now->cfl[0];
+    *mn = h->h_now->cfl[1];
     return FVM_OK;
 }
 
@@ -913,9 +948,7 @@ extern "C" int fvm_queue_dt(fvm_handle *h, const fvm_sim_params *p) {
     CHECK_INIT(h);
     if (!p) return set_err(FVM_ERR_INVALID, "null params");
     if (!h->cfl_valid) {
-        CK(launch_cfl_state(h->g, h->Un, h->mask, h->sc, h->stream));
-        h->launches++;
-        h->cfl_valid = true;
+        if (int r = queue_cfl(h)) return r;
     }
     CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
     h->launches_at_sc_copy = h->launches;
@@ -1285,6 +1318,7 @@ extern "C" int fvm_debug_stage1(fvm_handle *h, float dt, int with_ghost, float *
     CHECK_INIT(h);
     k_set_scalars<<<1, 1, 0, h->stream>>>(h->sc, dt, 0.0f, 0);
     h->launches_at_sc_copy = -1;
+    h->now_valid = false;
     CK(cudaGetLastError());
     float *Un = h->buf[BUF_N], *Us = h->buf[BUF_S];
     StepArgs a1 = step_args(h, Us, 1, 0, 1.0f);
@@ -1312,6 +1346,7 @@ extern "C" int fvm_debug_wait_timeout(fvm_handle *h, long long limit_cycles) {
     if (limit_cycles <= 0 || limit_cycles > kWaitCycles)
         return set_err(FVM_ERR_INVALID, "fvm_debug_wait_timeout: limit must be in 1..%lld cycles", kWaitCycles);
     CK(cudaStreamSynchronize(h->stream));
+    h->now_valid = false;
     CK(launch_wait_probe(h->sc, limit_cycles, h->stream));
     const int r = check_device_error(h);
     // clear the error word the probe set, so the solve goes on

@@ -3,6 +3,7 @@
 // reductions, velocity arrows, FP64 diagnostics and the shock standoff scan.
 #include <cstdint>
 
+#include "fvm_colortable.h"
 #include "fvm_kernels.cuh"
 #include "fvm_quads.cuh"
 #include "fvm_tma.cuh"
@@ -22,40 +23,89 @@ __global__ void k_primitives(GridDesc g, const float *U, float *u, float *v, flo
     if (T) T[d] = TT;
 }
 
-// The planes a derived field reads (derived_value): the others stay zero.
-template <int KIND>
+// The four cells a thread of a whole-field pass handles.  GROUP: a group of
+// four neighbours of a row, for destinations whose groups are 16-byte aligned.
+// Otherwise cells 32 apart in the dense order, so that a warp's loads and
+// stores are each 32 consecutive cells whatever the row length: four 4-byte
+// (16-byte) stores of neighbours per thread would leave each store of the warp
+// a quarter (half) of its sectors.
+template <bool GROUP>
+struct Cells4 {
+    size_t c[4], d[4];  // pitched and dense index
+    int n;              // cells inside the grid
+    __device__ __forceinline__ Cells4(const GridDesc &g, unsigned e) {
+        if (GROUP) {
+            const Quad q = quad_at(g, e);
+            n = q.n;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                c[k] = q.c + k;
+                d[k] = q.d + k;
+            }
+        } else {
+            const unsigned total = (unsigned)g.nx * (unsigned)g.ny, first = (e & ~31u) * 4u + (e & 31u);
+            unsigned j = first / (unsigned)g.nx, i = first - j * (unsigned)g.nx;
+            n = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned at = first + 32u * k;
+                n += at < total && at >= first ? 1 : 0;
+                c[k] = (size_t)j * g.pitch + i;
+                d[k] = at;
+                for (i += 32u; i >= (unsigned)g.nx; i -= (unsigned)g.nx) j++;
+            }
+        }
+    }
+    // threads that cover a grid
+    __host__ __device__ static unsigned threads(const GridDesc &g) {
+        return GROUP ? quads(g) : ((unsigned)g.nx * (unsigned)g.ny + 127u) / 128u * 32u;
+    }
+};
+
+// A derived field's inputs (derived_value): only the planes the kind reads, the
+// others zero.
+template <int KIND, bool GROUP>
 struct DerivedIn {
-    float4 rho, ru, rv, re;
-    __device__ __forceinline__ DerivedIn(const GridDesc &g, const float *U, const Quad &q) {
-        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        rho = KIND != 1 ? load4(U, q) : z;
-        ru = KIND >= 3 ? load4(U + g.plane, q) : z;
-        rv = KIND >= 3 ? load4(U + 2 * g.plane, q) : z;
-        re = KIND != 2 && KIND != 3 ? load4(U + 4 * g.plane, q) : z;
+    float rho[4], ru[4], rv[4], re[4];
+    __device__ __forceinline__ static void plane(float *dst, bool used, const float *p, const Cells4<GROUP> &q) {
+        if (GROUP) {
+            const float4 v = used ? __ldg(reinterpret_cast<const float4 *>(p + q.c[0])) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            dst[0] = v.x;
+            dst[1] = v.y;
+            dst[2] = v.z;
+            dst[3] = v.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) dst[k] = used && k < q.n ? __ldg(p + q.c[k]) : 0.0f;
+        }
     }
-    __device__ __forceinline__ float value(int k) const {
-        return derived_value(KIND, lane4(rho, k), lane4(ru, k), lane4(rv, k), lane4(re, k));
+    __device__ __forceinline__ DerivedIn(const GridDesc &g, const float *U, const Cells4<GROUP> &q) {
+        plane(rho, KIND != 1, U, q);
+        plane(ru, KIND >= 3, U + g.plane, q);
+        plane(rv, KIND >= 3, U + 2 * g.plane, q);
+        plane(re, KIND != 2 && KIND != 3, U + 4 * g.plane, q);
     }
+    __device__ __forceinline__ float value(int k) const { return derived_value(KIND, rho[k], ru[k], rv[k], re[k]); }
 };
 
 // Derived field into a dense nx*ny destination: 8 (density, pressure) to 20
 // (Mach) bytes per cell, DRAM-bound.  One launch per kind, so that only the
-// planes the kind needs are read.  VEC: every group's destination is 16-byte
-// aligned (nx a multiple of 4 and dst aligned).  Measured at 8192x4096,
-// all four planes read a cell at a time -> this: density and pressure 135 -> 39
-// us, temperature 135 -> 53, speed 135 -> 72, Mach 135 -> 92 (7.3 TB/s).
-template <int KIND, bool VEC>
+// planes the kind needs are read.  Measured at 8192x4096, all four planes read
+// a cell at a time -> this: density and pressure 135 -> 39 us, temperature
+// 135 -> 53, speed 135 -> 72, Mach 135 -> 92 (7.3 TB/s); at 4999x2501
+// density 53 -> 18, Mach 55 -> 41.
+template <int KIND, bool GROUP>
 __global__ void __launch_bounds__(256) k_derived(GridDesc g, const float *__restrict__ U, float *__restrict__ dst) {
     const unsigned e = blockIdx.x * 256u + threadIdx.x;
-    if (e >= quads(g)) return;
-    const Quad q = quad_at(g, e);
-    const DerivedIn<KIND> in(g, U, q);
-    if (VEC) {
-        *reinterpret_cast<float4 *>(dst + q.d) = make_float4(in.value(0), in.value(1), in.value(2), in.value(3));
+    if (e >= Cells4<GROUP>::threads(g)) return;
+    const Cells4<GROUP> q(g, e);
+    const DerivedIn<KIND, GROUP> in(g, U, q);
+    if (GROUP) {
+        *reinterpret_cast<float4 *>(dst + q.d[0]) = make_float4(in.value(0), in.value(1), in.value(2), in.value(3));
     } else {
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (k < q.n) dst[q.d + k] = in.value(k);
+            if (k < q.n) dst[q.d[k]] = in.value(k);
     }
 }
 
@@ -65,35 +115,47 @@ __device__ __forceinline__ float lerp_texel(float w, float a, float b) {
     return __fmaf_rn(w, b, __fmul_rn(1.0f - w, a));
 }
 
+// the tables in the order of enum fvm_colormap
+__device__ const ColormapLUT kColorTables[5] = {colormap_lut(0), colormap_lut(1), colormap_lut(2), colormap_lut(3),
+                                                colormap_lut(4)};
+
 // The renderer's field pass (FIELD_FRAGMENT_SHADER, src/renderer.cpp:47-77)
 // with one pixel per cell: SOLID and GHOST cells dark grey, others the
 // derived value normalised by (v - lo) / (hi - lo + 1e-4), clamped to [0, 1],
 // then looked up in the 256-entry colour table the way a linearly filtered,
 // edge-clamped 1-D texture samples it.  FMT 0: RGBA float, 1: RGBA8.
 // The table sits in shared memory as pairs of neighbouring entries, so a
-// lookup is two 16-byte loads; indexed in the kernel's parameters (constant
-// memory), lanes with different colours were served one after the other.
-// Mach -> RGBA8 at 8192x4096: 214 us that way, 132 us here (21 B per cell, 5.3
-// TB/s).
-template <int KIND, int FMT, bool VEC>
+// lookup is two vector loads; indexed in the kernel's parameters (constant
+// memory), lanes with different entries were served one after the other.
+// Mach -> RGBA8 at 8192x4096: 214 us indexed in constant memory, 112 us here
+// (21 B per cell, 6.3 TB/s); Mach -> RGBA float at 5000x2500 94 -> 71.
+template <int KIND, int FMT, bool GROUP>
 __global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__restrict__ U,
-                                                  const uint8_t *__restrict__ mask,
-                                                  const __grid_constant__ ColormapLUT lut, float lo, float hi,
-                                                  void *__restrict__ out) {
+                                                  const uint8_t *__restrict__ mask, int colormap, float lo,
+                                                  float hi, void *__restrict__ out) {
+    static_assert(!GROUP || FMT == 1, "groups of four only for 4-byte pixels");
     // entry i: {r_i, g_i, b_i, r_i+1}, {g_i+1, b_i+1, -, -}
     __shared__ float4 ta[256];
     __shared__ float2 tb[256];
     {
         const int i = threadIdx.x, n = min(i + 1, 255);
-        ta[i] = make_float4(lut.rgb[3 * i], lut.rgb[3 * i + 1], lut.rgb[3 * i + 2], lut.rgb[3 * n]);
-        tb[i] = make_float2(lut.rgb[3 * n + 1], lut.rgb[3 * n + 2]);
+        const float *rgb = kColorTables[colormap].rgb;
+        ta[i] = make_float4(rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2], rgb[3 * n]);
+        tb[i] = make_float2(rgb[3 * n + 1], rgb[3 * n + 2]);
     }
     __syncthreads();
-    const unsigned total = quads(g);
+    const unsigned total = Cells4<GROUP>::threads(g);
     for (unsigned e = blockIdx.x * 256u + threadIdx.x; e < total; e += gridDim.x * 256u) {
-        const Quad q = quad_at(g, e);
-        const DerivedIn<KIND> in(g, U, q);
-        const uint32_t m4 = __ldg(reinterpret_cast<const uint32_t *>(mask + q.c));
+        const Cells4<GROUP> q(g, e);
+        const DerivedIn<KIND, GROUP> in(g, U, q);
+        uint32_t m4 = 0u;  // mask bytes of the four cells
+        if (GROUP) {
+            m4 = __ldg(reinterpret_cast<const uint32_t *>(mask + q.c[0]));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k < q.n) m4 |= (uint32_t)__ldg(mask + q.c[k]) << (8 * k);
+        }
         float4 px[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -120,19 +182,20 @@ __global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__res
         if (FMT == 0) {
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                if (k < q.n) reinterpret_cast<float4 *>(out)[q.d + k] = px[k];
+                if (k < q.n) reinterpret_cast<float4 *>(out)[q.d[k]] = px[k];
         } else {
             auto quant = [](float x) { return (unsigned)__float2int_rn(fminf(fmaxf(x, 0.0f), 1.0f) * 255.0f); };
             uint32_t w[4];
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 w[k] = quant(px[k].x) | (quant(px[k].y) << 8) | (quant(px[k].z) << 16) | (255u << 24);
-            if (VEC) {
-                *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(out) + q.d) = make_uint4(w[0], w[1], w[2], w[3]);
+            uint32_t *const o = reinterpret_cast<uint32_t *>(out);
+            if (GROUP) {
+                *reinterpret_cast<uint4 *>(o + q.d[0]) = make_uint4(w[0], w[1], w[2], w[3]);
             } else {
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    if (k < q.n) reinterpret_cast<uint32_t *>(out)[q.d + k] = w[k];
+                    if (k < q.n) o[q.d[k]] = w[k];
             }
         }
     }
@@ -486,27 +549,32 @@ static bool dense_aligned(const GridDesc &g, const void *p) {
     return (g.nx & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
 }
 
-template <int KIND>
-static void colormap_k(const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut, float lo,
-                       float hi, void *out, int fmt, cudaStream_t st) {
-    // enough blocks to fill the chip several times over, each filling its table once
-    const unsigned nb = quad_blocks(g, 148 * 32);
-    if (fmt == 0)
-        k_colormap<KIND, 0, false><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
-    else if (dense_aligned(g, out))
-        k_colormap<KIND, 1, true><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
-    else
-        k_colormap<KIND, 1, false><<<nb, 256, 0, st>>>(g, U, mask, lut, lo, hi, out);
+template <bool GROUP>
+static unsigned cell_blocks(const GridDesc &g) {
+    return (Cells4<GROUP>::threads(g) + 255u) / 256u;
 }
 
-cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut,
+template <int KIND>
+static void colormap_k(const GridDesc &g, const float *U, const uint8_t *mask, int colormap, float lo,
+                       float hi, void *out, int fmt, cudaStream_t st) {
+    // enough blocks to fill the chip several times over, each filling its table once
+    constexpr unsigned kCap = 148 * 32;
+    if (fmt == 0)
+        k_colormap<KIND, 0, false><<<std::min(kCap, cell_blocks<false>(g)), 256, 0, st>>>(g, U, mask, colormap, lo, hi, out);
+    else if (dense_aligned(g, out))
+        k_colormap<KIND, 1, true><<<std::min(kCap, cell_blocks<true>(g)), 256, 0, st>>>(g, U, mask, colormap, lo, hi, out);
+    else
+        k_colormap<KIND, 1, false><<<std::min(kCap, cell_blocks<false>(g)), 256, 0, st>>>(g, U, mask, colormap, lo, hi, out);
+}
+
+cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, int colormap,
                             float lo, float hi, void *out, int fmt, cudaStream_t st) {
     switch (kind) {
-    case 0: colormap_k<0>(g, U, mask, lut, lo, hi, out, fmt, st); break;
-    case 1: colormap_k<1>(g, U, mask, lut, lo, hi, out, fmt, st); break;
-    case 2: colormap_k<2>(g, U, mask, lut, lo, hi, out, fmt, st); break;
-    case 3: colormap_k<3>(g, U, mask, lut, lo, hi, out, fmt, st); break;
-    default: colormap_k<4>(g, U, mask, lut, lo, hi, out, fmt, st); break;
+    case 0: colormap_k<0>(g, U, mask, colormap, lo, hi, out, fmt, st); break;
+    case 1: colormap_k<1>(g, U, mask, colormap, lo, hi, out, fmt, st); break;
+    case 2: colormap_k<2>(g, U, mask, colormap, lo, hi, out, fmt, st); break;
+    case 3: colormap_k<3>(g, U, mask, colormap, lo, hi, out, fmt, st); break;
+    default: colormap_k<4>(g, U, mask, colormap, lo, hi, out, fmt, st); break;
     }
     return cudaGetLastError();
 }
@@ -514,9 +582,9 @@ cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const u
 template <int KIND>
 static void derived_k(const GridDesc &g, const float *U, float *dst, cudaStream_t st) {
     if (dense_aligned(g, dst))
-        k_derived<KIND, true><<<quad_blocks(g), 256, 0, st>>>(g, U, dst);
+        k_derived<KIND, true><<<cell_blocks<true>(g), 256, 0, st>>>(g, U, dst);
     else
-        k_derived<KIND, false><<<quad_blocks(g), 256, 0, st>>>(g, U, dst);
+        k_derived<KIND, false><<<cell_blocks<false>(g), 256, 0, st>>>(g, U, dst);
 }
 
 cudaError_t launch_derived(int kind, const GridDesc &g, const float *U, float *dst, cudaStream_t st) {

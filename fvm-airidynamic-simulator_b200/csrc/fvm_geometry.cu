@@ -7,6 +7,7 @@
 // classes come out bit-identical.
 #include "fvm_internal.cuh"
 #include "fvm_kernels.cuh"
+#include "fvm_quads.cuh"
 
 namespace fvm {
 
@@ -236,32 +237,50 @@ __global__ void k_sdf(GridDesc g, ShapeArgs s, float *sdf, uint8_t *ct, float *f
 
 __device__ __forceinline__ bool is_wall_ct(uint8_t t) { return t == CT_SOLID || t == CT_GHOST; }
 
-// Mask byte of each cell (see fvm_math.cuh), from the dense cell classes.
-__global__ void k_mask(GridDesc g, const uint8_t *ct, uint8_t *mask) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
+// Mask byte of each cell (see fvm_math.cuh), from the dense cell classes: four
+// cells of a row per thread, whose 3 + 4 + 4 x 4 classes are read once each
+// where a cell on its own reads nine, and whose bytes are one store.
+// 8192x4096: 169 us one cell per thread, 104 us here.
+__global__ void __launch_bounds__(256) k_mask(GridDesc g, const uint8_t *__restrict__ ct, uint8_t *__restrict__ mask) {
+    const unsigned e = blockIdx.x * 256u + threadIdx.x;
+    if (e >= quads(g)) return;
+    const Quad q = quad_at(g, e);
     const int nx = g.nx, ny = g.ny;
-    auto at = [&](int ii, int jj) {
-        ii = max(0, min(ii, nx - 1));
-        jj = max(0, min(jj, ny - 1));
-        return ct[(size_t)jj * nx + ii];
-    };
-    uint8_t t = at(i, j);
-    uint32_t m = (uint32_t)t << MB_TYPE_SHIFT;
-    if (is_wall_ct(t)) m |= MB_WALL;
-    if (i < nx - 1) {
-        if (!is_wall_ct(t) && !is_wall_ct(at(i + 1, j))) m |= MB_XV;
-        if (is_wall_ct(at(i - 1, j)) || is_wall_ct(at(i + 2, j))) m |= MB_XN;
+    // wall flags of columns q.i-1 .. q.i+5 of row j, edge cells repeated
+    const uint8_t *row = ct + (size_t)q.j * nx;
+    uint8_t t[4];
+    bool w[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        const uint8_t c = row[max(0, min(q.i - 1 + k, nx - 1))];
+        if (k >= 1 && k <= 4) t[k - 1] = c;
+        w[k] = is_wall_ct(c);
     }
-    if (j < ny - 1) {
-        if (!is_wall_ct(t) && !is_wall_ct(at(i, j + 1))) m |= MB_YV;
-        if (is_wall_ct(at(i, j - 1)) || is_wall_ct(at(i, j + 2))) m |= MB_YN;
+    const uint8_t *below = ct + (size_t)max(q.j - 1, 0) * nx, *above = ct + (size_t)min(q.j + 1, ny - 1) * nx,
+                  *above2 = ct + (size_t)min(q.j + 2, ny - 1) * nx;
+    uint32_t word = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = q.i + k;
+        if (k >= q.n) break;
+        uint32_t m = (uint32_t)t[k] << MB_TYPE_SHIFT;
+        if (w[k + 1]) m |= MB_WALL;
+        if (i < nx - 1) {
+            if (!w[k + 1] && !w[k + 2]) m |= MB_XV;
+            if (w[k] || w[k + 3]) m |= MB_XN;
+        }
+        if (q.j < ny - 1) {
+            if (!w[k + 1] && !is_wall_ct(above[i])) m |= MB_YV;
+            if (is_wall_ct(below[i]) || is_wall_ct(above2[i])) m |= MB_YN;
+        }
+        word |= m << (8 * k);
     }
-    mask[(size_t)j * g.pitch + i] = (uint8_t)m;
+    // the row's padding may take the bytes beyond nx
+    *reinterpret_cast<uint32_t *>(mask + q.c) = word;
 }
 
-// Ghost-cell table: count pass (list == nullptr) or fill pass.
+// Ghost-cell table: fills `list` up to its capacity and counts every ghost cell
+// (a count pass alone with list == nullptr).
 // Normal and neighbour dot products use the reference's expressions
 // (src/solver.cu:2054-2098); a candidate must have sdf > 0 and dot > -1 (the
 // reference's initial best_dot), its density is checked at run time.
@@ -349,8 +368,7 @@ void launch_sdf(const GridDesc &g, const ShapeParamsHost &s, float *sdf, uint8_t
 }
 
 void launch_mask(const GridDesc &g, const uint8_t *ct, uint8_t *mask, cudaStream_t st) {
-    dim3 b(32, 8);
-    k_mask<<<grid2d(g, b), b, 0, st>>>(g, ct, mask);
+    k_mask<<<quad_blocks(g), 256, 0, st>>>(g, ct, mask);
 }
 
 void launch_ghost_table(const GridDesc &g, const float *sdf, const uint8_t *ct, GhostInfo *list, int cap, int *count,

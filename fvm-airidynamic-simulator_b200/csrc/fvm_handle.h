@@ -40,6 +40,10 @@ struct fvm_handle {
     DevScalars *sc = nullptr;
     DevScalars *h_sc = nullptr;  // pinned mirror
     float *d_tmp = nullptr;      // reduction scratch: {maximum, counter} of the max pass, counter of the diagnostics
+    HostScalars *h_now = nullptr;  // the scalars as kernels write them to the host (behind h_res, pinned)
+    // h_now (once the stream is idle) holds the last step's or CFL pass's scalars:
+    // no later kernel changed what it mirrors
+    bool now_valid = false;
     double *h_res = nullptr;     // 8 results the reduction kernels write to the host (behind h_sc, pinned)
     int *d_counter = nullptr;    // arrows counter
     double *d_diag = nullptr;    // partials of the diagnostics

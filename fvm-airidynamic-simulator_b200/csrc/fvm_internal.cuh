@@ -50,6 +50,16 @@ struct DevScalars {
     double diag[16];  // FP64 diagnostic accumulators
 };
 
+// What the host reads back of a solve's scalars, in pinned host memory: the last
+// block of a call's final ghost pass (and of the CFL pass) writes it, so the
+// host needs no copy, only the stream's completion.
+struct HostScalars {
+    float cfl[2];
+    float dt_last, t;
+    unsigned err;
+    unsigned pad;
+};
+
 // compute{Temperature,Pressure,VelocityMag,Mach}DirectKernel and the density
 // copy (src/solver.cu:3527-3671): the derived value of one cell (kind =
 // FVM_FIELD_*).  Used by the derived-field pass and, for a registered display
@@ -121,6 +131,7 @@ struct GhostArgs {
     float cfl_num, cfl_visc, min_dx;
     int viscous;
     int flip_parity;       // batched solves: toggle sc->parity in the finalize
+    HostScalars *host;     // finalize: the scalars' copy on the host, or null
     const DisplayDesc *disp;  // display field of the ghost cells written (dense nx*ny), or null
 };
 

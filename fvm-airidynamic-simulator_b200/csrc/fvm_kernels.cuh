@@ -56,11 +56,14 @@ cudaError_t launch_set_display(DisplayDesc *d, float *ptr, int kind, cudaStream_
 cudaError_t launch_ghost(const GhostArgs &a, cudaStream_t st);
 // Bounded wait on an mbarrier nothing arrives on (expires after limit_cycles).
 cudaError_t launch_wait_probe(DevScalars *sc, long long limit_cycles, cudaStream_t st);
-// Phase-1 boundary conditions in place on a whole state (set-up path).
-cudaError_t launch_bc_phase1(const GridDesc &g, float *U, const uint8_t *mask, const Freestream &fs, cudaStream_t st);
+// Phase-1 boundary conditions in place on a whole state (set-up path); the
+// ghost cells' state goes to `snap` (a state buffer; null: not kept).
+cudaError_t launch_bc_phase1(const GridDesc &g, float *U, const uint8_t *mask, const Freestream &fs, float *snap,
+                             cudaStream_t st);
 // CFL maxima of a state (speed over all cells; nu = mu(T)/rho, mu = 0 in solids),
 // published to sc->cfl by the last block (sc->red and sc->counter are zero before and after).
-cudaError_t launch_cfl_state(const GridDesc &g, const float *U, const uint8_t *mask, DevScalars *sc, cudaStream_t st);
+cudaError_t launch_cfl_state(const GridDesc &g, const float *U, const uint8_t *mask, DevScalars *sc, HostScalars *host,
+                             cudaStream_t st);
 // Set the dynamic shared-memory attribute of every step kernel of a tuning.
 cudaError_t prepare_step_kernels(const StageTune &tn);
 // Shared-memory bytes a stage / viscous kernel needs for a tuning.
@@ -74,12 +77,12 @@ int stage_box_blend(const StageTune &tn);      // TMA box width of the blend par
 cudaError_t launch_primitives(const GridDesc &g, const float *U, float *u, float *v, float *p, float *T,
                               cudaStream_t st);  // dense nx*ny outputs
 cudaError_t launch_derived(int kind, const GridDesc &g, const float *U, float *dst, cudaStream_t st);
-// 256-entry RGB colour table, passed to the kernel by value.
+// 256-entry RGB colour table.
 struct ColormapLUT {
     float rgb[256 * 3];
 };
 // mask: the pitched mask bytes (their wall bit marks SOLID and GHOST cells)
-cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, const ColormapLUT &lut,
+cudaError_t launch_colormap(int kind, const GridDesc &g, const float *U, const uint8_t *mask, int colormap,
                             float lo, float hi, void *out, int fmt, cudaStream_t st);
 cudaError_t launch_ct_to_float(const GridDesc &g, const uint8_t *ct, float *dst, cudaStream_t st);
 // The results of the next three go to pinned host memory (out_host), valid once

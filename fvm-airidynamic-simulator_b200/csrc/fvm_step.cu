@@ -1127,6 +1127,13 @@ __device__ void finalize_cfl(const GhostArgs &a) {
     red[0] = 0.0f;
     red[1] = 0.0f;
     if (a.flip_parity) sc->parity ^= 1u;
+    if (a.host) {  // visible to the host when the kernel has completed
+        a.host->cfl[0] = ms;
+        a.host->cfl[1] = mn;
+        a.host->dt_last = sc->dt_last;
+        a.host->t = sc->t;
+        a.host->err = *reinterpret_cast<volatile unsigned *>(&sc->err);
+    }
     __threadfence();
     sc->counter = 0;
 }
@@ -1263,23 +1270,39 @@ __global__ void __launch_bounds__(128) k_ghost_batch(const BatchInst *__restrict
     ghost_publish(a, ls, ln, nbad, (unsigned)I.n_gchunks);
 }
 
-// Phase-1 boundary conditions in place (set-up path).
-__global__ void k_bc_phase1(GridDesc g, float *U, const uint8_t *mask, Freestream fs) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    size_t c = (size_t)j * g.pitch + i;
-    float s[5];
-    for (int k = 0; k < 5; k++) s[k] = U[k * g.plane + c];
-    bc_pointwise(s, mb_type(mask[c]), i, j, g.nx, g.ny, fs);
-    for (int k = 0; k < 5; k++) U[k * g.plane + c] = s[k];
+// Phase-1 boundary conditions in place (set-up path).  They act on non-fluid
+// cells and the domain's edge cells only, so the others cost their mask byte.
+// Ghost cells, which phase 1 leaves alone, are copied to `snap`: the ghost pass
+// reads their pre-call values there (instead of from a copy of the whole state).
+// 8192x4096: 224 us and the copy before, 62 us here.
+__global__ void __launch_bounds__(256) k_bc_phase1(GridDesc g, float *U, const uint8_t *__restrict__ mask, Freestream fs,
+                                                   float *snap) {
+    const unsigned e = blockIdx.x * 256u + threadIdx.x;
+    if (e >= quads(g)) return;
+    const Quad q = quad_at(g, e);
+    const uint32_t m4 = *reinterpret_cast<const uint32_t *>(mask + q.c);
+    const bool edge_row = q.j == 0 || q.j == g.ny - 1;
+#pragma unroll 1
+    for (int k = 0; k < q.n; k++) {
+        const uint32_t type = mb_type(m4 >> (8 * k));
+        const int i = q.i + k;
+        if (type == CT_FLUID && !edge_row && i != 0 && i != g.nx - 1) continue;
+        const size_t c = q.c + k;
+        float s[5];
+        for (int f = 0; f < 5; f++) s[f] = U[f * g.plane + c];
+        if (type == CT_GHOST && snap)
+            for (int f = 0; f < 5; f++) snap[f * g.plane + c] = s[f];
+        bc_pointwise(s, type, i, q.j, g.nx, g.ny, fs);
+        for (int f = 0; f < 5; f++) U[f * g.plane + c] = s[f];
+    }
 }
 
 // CFL maxima of a whole state (computeWaveSpeedKernel / computeViscousNumberKernel);
 // the last block publishes them and leaves the accumulators zero.  20 B of
 // state and 1 B of mask per cell in 16-byte loads: 112 us
 // at 8192x4096 (202 us plus a publishing kernel when read a cell at a time).
-__global__ void __launch_bounds__(256, 6) k_cfl_state(GridDesc g, const float *U, const uint8_t *mask, DevScalars *sc) {
+__global__ void __launch_bounds__(256, 6) k_cfl_state(GridDesc g, const float *U, const uint8_t *mask, DevScalars *sc,
+                                                      HostScalars *host) {
     float ls = 0.0f, ln = 0.0f;
     const unsigned total = quads(g);
     for (unsigned e = blockIdx.x * 256u + threadIdx.x; e < total; e += gridDim.x * 256u) {
@@ -1303,8 +1326,11 @@ __global__ void __launch_bounds__(256, 6) k_cfl_state(GridDesc g, const float *U
     }
     block_max2_publish<256>(ls, ln, sc->red);
     if (last_block(&sc->counter) && threadIdx.x == 0) {
-        sc->cfl[0] = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(&sc->red[0]), 0u));
-        sc->cfl[1] = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(&sc->red[1]), 0u));
+        host->cfl[0] = sc->cfl[0] = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(&sc->red[0]), 0u));
+        host->cfl[1] = sc->cfl[1] = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(&sc->red[1]), 0u));
+        host->dt_last = sc->dt_last;
+        host->t = sc->t;
+        host->err = sc->err;
     }
 }
 
@@ -1585,14 +1611,15 @@ cudaError_t launch_ghost(const GhostArgs &a, cudaStream_t st) {
     return launch_step_kernel(true, k_ghost, dim3(blocks), dim3(128), 0, st, a);
 }
 
-cudaError_t launch_bc_phase1(const GridDesc &g, float *U, const uint8_t *mask, const Freestream &fs, cudaStream_t st) {
-    dim3 b(32, 8), gr((g.nx + 31) / 32, (g.ny + 7) / 8);
-    k_bc_phase1<<<gr, b, 0, st>>>(g, U, mask, fs);
+cudaError_t launch_bc_phase1(const GridDesc &g, float *U, const uint8_t *mask, const Freestream &fs, float *snap,
+                             cudaStream_t st) {
+    k_bc_phase1<<<quad_blocks(g), 256, 0, st>>>(g, U, mask, fs, snap);
     return cudaGetLastError();
 }
 
-cudaError_t launch_cfl_state(const GridDesc &g, const float *U, const uint8_t *mask, DevScalars *sc, cudaStream_t st) {
-    k_cfl_state<<<quad_blocks(g, 148 * 6), 256, 0, st>>>(g, U, mask, sc);
+cudaError_t launch_cfl_state(const GridDesc &g, const float *U, const uint8_t *mask, DevScalars *sc, HostScalars *host,
+                             cudaStream_t st) {
+    k_cfl_state<<<quad_blocks(g, 148 * 6), 256, 0, st>>>(g, U, mask, sc, host);
     return cudaGetLastError();
 }
 
