@@ -463,11 +463,9 @@ extern "C" int fvm_batch_read_fields(fvm_batch *b, int id, float *rho, float *rh
     unsigned parity = 0;
     BCK(cudaMemcpy(&parity, &h->sc->parity, sizeof parity, cudaMemcpyDeviceToHost));
     const float *src = h->buf[parity ? BUF_X : BUF_N];
-    float *dst[5] = {rho, rho_u, rho_v, E, rho_e};
-    for (int k = 0; k < 5; k++)
-        if (dst[k])
-            BCK(cudaMemcpy2D(dst[k], (size_t)h->g.nx * 4, src + (size_t)k * h->g.plane, (size_t)h->g.pitch * 4,
-                             (size_t)h->g.nx * 4, h->g.ny, cudaMemcpyDeviceToHost));
+    float *const dst[5] = {rho, rho_u, rho_v, E, rho_e};
+    if (int r = fvm_internal_copy_fields(h->g, src, dst, b->stream)) return r;
+    BCK(cudaStreamSynchronize(b->stream));
     return FVM_OK;
 }
 

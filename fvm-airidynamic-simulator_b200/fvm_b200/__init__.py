@@ -159,6 +159,13 @@ def _p(a):
     return C.c_void_p(a.ctypes.data) if a is not None else None
 
 
+def _planes(k, *shape):
+    """(array, pointers): k float32 planes of `shape` in one array, which the
+    library then fills with one copy instead of k arrays to be stacked after."""
+    a = np.empty((k,) + shape, np.float32)
+    return a, [C.c_void_p(a.ctypes.data + i * a.strides[0]) for i in range(k)]
+
+
 class Solver:
     """One solve on the GPU (the reference CFDSolver's public surface)."""
 
@@ -232,16 +239,15 @@ class Solver:
 
     # readback --------------------------------------------------------------
     def fields(self):
-        n = self.params.nx * self.params.ny
-        out = [np.empty(n, np.float32) for _ in range(5)]
-        _check(self.lib.fvm_read_fields(self.h, *[_p(a) for a in out]))
-        return np.stack([a.reshape(self.shape) for a in out])
+        out, ptrs = _planes(5, *self.shape)
+        _check(self.lib.fvm_read_fields(self.h, *ptrs))
+        return out
 
     def read_region(self, i0, j0, w, h):
         """Conserved fields of the window [i0, i0+w) x [j0, j0+h): (5, h, w) float32."""
-        out = [np.empty(w * h, np.float32) for _ in range(5)]
-        _check(self.lib.fvm_read_region(self.h, int(i0), int(j0), int(w), int(h), *[_p(a) for a in out]))
-        return np.stack([a.reshape(h, w) for a in out])
+        out, ptrs = _planes(5, h, w)
+        _check(self.lib.fvm_read_region(self.h, int(i0), int(j0), int(w), int(h), *ptrs))
+        return out
 
     def read_region_geometry(self, i0, j0, w, h):
         """(sdf float32 (h, w), cell classes uint8 (h, w)) of the window."""
@@ -255,10 +261,9 @@ class Solver:
         _check(self.lib.fvm_write_fields(self.h, *[_p(a) for a in U]))
 
     def primitives(self):
-        n = self.params.nx * self.params.ny
-        out = [np.empty(n, np.float32) for _ in range(4)]
-        _check(self.lib.fvm_read_primitives(self.h, *[_p(a) for a in out]))
-        return np.stack([a.reshape(self.shape) for a in out])
+        out, ptrs = _planes(4, *self.shape)
+        _check(self.lib.fvm_read_primitives(self.h, *ptrs))
+        return out
 
     def cell_types(self):
         out = np.empty(self.params.nx * self.params.ny, np.uint8)
@@ -443,10 +448,9 @@ class Batch:
         return p
 
     def fields(self, id_):
-        ny, nx = self.shapes[id_]
-        out = [np.empty(nx * ny, np.float32) for _ in range(5)]
-        _check(self.lib.fvm_batch_read_fields(self.h, int(id_), *[_p(a) for a in out]))
-        return np.stack([a.reshape(ny, nx) for a in out])
+        out, ptrs = _planes(5, *self.shapes[id_])
+        _check(self.lib.fvm_batch_read_fields(self.h, int(id_), *ptrs))
+        return out
 
     def diagnostics(self, id_):
         d = Diag()
@@ -501,8 +505,7 @@ class Server:
         """Queue a solve of `steps` steps; returns its ticket."""
         t = C.c_longlong()
         if keep_fields:
-            arrs = [np.empty((params.ny, params.nx), np.float32) for _ in range(5)]
-            ptrs = [_p(a) for a in arrs]
+            arrs, ptrs = _planes(5, params.ny, params.nx)
         else:
             arrs, ptrs = None, [None] * 5
         _check(self.lib.fvm_server_submit(self.h, C.byref(params), int(steps), *ptrs, C.byref(t)))
@@ -511,7 +514,7 @@ class Server:
 
     def _collect(self, r):
         arrs = self.outputs.pop(r.ticket, None)
-        fields = np.stack(arrs) if arrs is not None and r.status == 0 else None
+        fields = arrs if arrs is not None and r.status == 0 else None
         return r, fields
 
     def wait(self, ticket, timeout_s=-1.0):
