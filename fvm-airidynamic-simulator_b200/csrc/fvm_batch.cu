@@ -33,6 +33,7 @@ struct fvm_batch {
     GhostChunk *d_chunks = nullptr;
     int n_active = 0, n_stage_tiles = 0, n_visc_tiles = 0, n_chunks = 0;
     size_t cap_insts = 0, cap_stage = 0, cap_visc = 0, cap_chunks = 0;
+    bool flat = false;                // stages on flat tiles (d_stage_tiles lists those then)
     bool dirty = true;
     cudaGraphExec_t graph = nullptr;
     long long launches = 0;
@@ -65,18 +66,36 @@ static int ensure(T **ptr, size_t *cap, size_t n) {
 // Rows per tile for the current set of instances: the tallest tile in
 // {64, 32, 16} that still gives about 2000 tiles, so the persistent grid
 // (148 SMs x resident CTAs) stays fed with work while tall tiles keep the
-// per-tile halo rows cheap.  Measured on B200: 48M cells over 256 solves run
-// best at 64, ~10M cells at 32, ~2.7M cells at 16 (64 loses 16 % there).
+// per-tile halo rows cheap; for small batches the tallest of {16, 8} that gives
+// every resident CTA a tile, else 4.  Measured on B200: 48M cells over 256
+// solves run best at 64, ~10M cells at 32, ~2.7M cells at 16 (64 loses 16 %
+// there), 4 solves of 128x64 43 us a step at 4 rows against 84 at 16.
 static int batch_rows(const fvm_batch *b) {
     const int W = stage_cols_per_cta(b->tune);
-    for (int rows : {64, 32}) {
+    for (int rows : {64, 32, 16, 8}) {
         long long tiles = 0;
         for (const fvm_handle *h : b->slots)
             if (h) tiles += (long long)((h->g.nx + W - 1) / W) * ((h->g.ny + rows - 1) / rows);
-        if (tiles >= 2000) return rows;
+        if (tiles >= (rows > 16 ? 2000 : 740)) return rows;
     }
-    return 16;
+    return 4;
 }
+
+static long long batch_cells(const fvm_batch *b) {
+    long long n = 0;
+    for (const fvm_handle *h : b->slots)
+        if (h) n += (long long)h->g.nx * h->g.ny;
+    return n;
+}
+
+// Cells up to which a batch's stages run on flat tiles.  The limit is higher than
+// a single solve's: the persistent marching stages keep their arguments in
+// shared memory and run 5 CTAs per SM with spills, and the narrow grids of a
+// batch fill their 124-column strips badly.  Measured steps, marching -> flat:
+// 16 solves 0.3M cells 81.9 -> 65.2 us, 1.5M 178.9 -> 151.2, 64 solves 9.1M
+// 724 -> 698, 11.8M 920 -> 884, 128 solves 22.7M 1617 -> 1645, 256 solves 43.9M
+// 3208 -> 3202 us.
+constexpr long long kBatchFlatCells = 16000000;
 
 // Rebuild the device descriptors and tile lists after the set of instances changed.
 static int rebuild(fvm_batch *b) {
@@ -85,6 +104,7 @@ static int rebuild(fvm_batch *b) {
     std::vector<GhostChunk> chunks;
     if (!b->tune_fixed) b->tune.rows = batch_rows(b);
     const int W = stage_cols_per_cta(b->tune), rows = b->tune.rows;
+    b->flat = !b->tune_fixed && batch_cells(b) <= kBatchFlatCells;
     for (size_t id = 0; id < b->slots.size(); id++) {
         fvm_handle *h = b->slots[id];
         if (!h) continue;
@@ -112,11 +132,15 @@ static int rebuild(fvm_batch *b) {
         I.min_dx = fminf(h->prm.dx, h->prm.dy);
         const int inst = (int)insts.size();
         insts.push_back(I);
-        for (int j0 = 0; j0 < h->g.ny; j0 += rows)
-            for (int i0 = 0; i0 < h->g.nx; i0 += W) {
-                stiles.push_back(TileDesc{inst, i0, j0, 0});
-                if (I.viscous) vtiles.push_back(TileDesc{inst, i0, j0, 0});
-            }
+        auto tile_list = [&](std::vector<TileDesc> &list, int height, int width) {
+            for (int j0 = 0; j0 < h->g.ny; j0 += height)
+                for (int i0 = 0; i0 < h->g.nx; i0 += width) list.push_back(TileDesc{inst, i0, j0, 0});
+        };
+        if (b->flat)
+            tile_list(stiles, 2 * kBatchFlatPairs, kBatchFlatCols);
+        else
+            tile_list(stiles, rows, W);
+        if (I.viscous) tile_list(vtiles, rows, W);
         for (int c = 0; c < I.n_gchunks; c++) chunks.push_back(GhostChunk{inst, c * 128, 128, 0});
     }
     if (int r = ensure(&b->d_insts, &b->cap_insts, insts.size())) return r;
@@ -157,9 +181,14 @@ static int enqueue_batch_step(fvm_batch *b) {
     // let the ghost pass after them launch early; with viscous instances the
     // post half step follows stage 2, which then launches plainly
     const bool visc = b->n_visc_tiles > 0;
-    BCK(launch_stage_batch(1, sch, lim, tn, b->d_insts, b->d_stage_tiles, b->n_stage_tiles, 1, true, st));
+    auto stage = [&](int which, int early, bool pdl) {
+        if (b->flat)
+            return launch_stage_flat_batch(which, sch, lim, b->d_insts, b->d_stage_tiles, b->n_stage_tiles, early, pdl, st);
+        return launch_stage_batch(which, sch, lim, tn, b->d_insts, b->d_stage_tiles, b->n_stage_tiles, early, pdl, st);
+    };
+    BCK(stage(1, 1, true));
     BCK(launch_ghost_batch(b->d_insts, b->d_chunks, b->n_chunks, 1, st));
-    BCK(launch_stage_batch(2, sch, lim, tn, b->d_insts, b->d_stage_tiles, b->n_stage_tiles, visc ? 0 : 1, !visc, st));
+    BCK(stage(2, visc ? 0 : 1, !visc));
     b->launches += 3;
     if (b->n_visc_tiles) {
         BCK(launch_viscous_batch(tn, b->d_insts, b->d_visc_tiles, b->n_visc_tiles, 1, st));

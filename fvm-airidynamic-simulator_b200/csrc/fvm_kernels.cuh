@@ -47,6 +47,10 @@ cudaError_t launch_viscous(const StageTune &tn, const CUtensorMap &tm_in, const 
 // follows); pdl: launch with programmatic stream serialization
 cudaError_t launch_stage_batch(int stage, int scheme, int limiter, const StageTune &tn, const BatchInst *insts,
                                const TileDesc *tiles, int ntiles, int early, bool pdl, cudaStream_t st);
+// The same stages on flat tiles of 32 x 2*kBatchFlatPairs cells.
+constexpr int kBatchFlatPairs = 7, kBatchFlatCols = 32;
+cudaError_t launch_stage_flat_batch(int stage, int scheme, int limiter, const BatchInst *insts, const TileDesc *tiles,
+                                    int ntiles, int early, bool pdl, cudaStream_t st);
 cudaError_t launch_viscous_batch(const StageTune &tn, const BatchInst *insts, const TileDesc *tiles, int ntiles,
                                  int post, cudaStream_t st);
 cudaError_t launch_ghost_batch(const BatchInst *insts, const GhostChunk *chunks, int nchunks, int mode,

@@ -483,9 +483,10 @@ __device__ __forceinline__ bool stage_tile(const CUtensorMap *tm_in, const CUten
     return true;
 }
 
-// Occupancy target: 6 CTAs of 128 threads per SM (80 registers, no spills;
-// ~30 KB of shared memory per CTA for stage 1, ~35 KB for stage 2 with its
-// blend pair).
+// Occupancy target: 6 CTAs of 128 threads per SM (80 registers; none to 8 bytes
+// of spills with HLLC, up to 24 with AUSM+; at 5 CTAs and no spills the HLLC
+// stages were 2 % slower; ~30 KB of shared memory per CTA for stage 1, ~35 KB
+// for stage 2 with its blend pair).
 template <int NT, int K, int STAGE, int SCHEME, int LIM, bool DISP>
 __global__ void __launch_bounds__(NT, 768 / NT)
     k_stage(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_blend,
@@ -539,21 +540,26 @@ struct FlatTile {
     static constexpr int THREADS = X * (PAIRS + 1);
     static constexpr int COLS = X + 4, SLOTS = PAIRS + 2;
     static_assert(THREADS >= PAIRS * (X + 1), "one x-face pair per thread");
+    struct Smem {
+        float4 PA[SLOTS][COLS], PB[SLOTS][COLS];                       // primitives of row pairs
+        float4 XA[PAIRS][X + 1], XB[PAIRS][X + 1], XC[PAIRS][X + 1];  // x-faces
+        float YU[6][PAIRS][X];  // upper y-face of pair p-1: fluxes and face velocity
+        uint16_t M[SLOTS][COLS];
+    };
 };
 
+// The tile at (i0, j0): everything but the launch order and the reductions.
 template <int PAIRS, int STAGE, int SCHEME, int LIM, bool DISP>
-__global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIRS>::THREADS)
-    k_stage_flat(const StepArgs a, const float *in, const float *blend) {
+__device__ __forceinline__ void flat_tile(const StepArgs &a, const float *in, const float *blend, int i0, int j0,
+                                          typename FlatTile<PAIRS>::Smem &sm, float &lmax, unsigned &nbad) {
     using L = FlatTile<PAIRS>;
-    __shared__ float4 PA[L::SLOTS][L::COLS], PB[L::SLOTS][L::COLS];
-    __shared__ float4 XA[PAIRS][L::X + 1], XB[PAIRS][L::X + 1], XC[PAIRS][L::X + 1];
-    __shared__ float YU[6][PAIRS][L::X];  // upper y-face of pair p-1: fluxes and face velocity
-    __shared__ uint16_t M[L::SLOTS][L::COLS];
+    auto &PA = sm.PA, &PB = sm.PB;
+    auto &XA = sm.XA, &XB = sm.XB, &XC = sm.XC;
+    auto &YU = sm.YU;
+    auto &M = sm.M;
     const GridDesc &g = a.g;
     const int nx = g.nx, ny = g.ny;
     const int t = threadIdx.x;
-    const int i0 = blockIdx.x * L::X, j0 = blockIdx.y * L::ROWS;
-    pdl_wait();
     const UpdateArgs ua{a.sc->dt * a.dt_scale, 1.0f / g.dx, 1.0f / g.dy};
     for (int k = t; k < L::SLOTS * L::COLS; k += L::THREADS) {
         const int s = k / L::COLS, x = k - s * L::COLS;
@@ -616,8 +622,6 @@ __global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIR
         YU[5][p + 1][c] = vfy.y;
     }
     __syncthreads();
-    float lmax = 0.0f;
-    unsigned nbad = 0;
     const int iu = i0 + c, u0 = j0 + 2 * p;
     if (p >= 0 && iu < nx && u0 < ny) {
         const bool st1 = u0 + 1 < ny;
@@ -640,6 +644,17 @@ __global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIR
             a, ua, M[p + 1][c + 2], iu, u0, true, st1, iu == 0 || iu == nx - 1, Uc, dX, dY, du, dv, mk2(B1.z, B1.w),
             [&](int k) { return mk2(blend[k * g.plane + cell], blend[k * g.plane + up]); }, lmax, nbad);
     }
+}
+
+template <int PAIRS, int STAGE, int SCHEME, int LIM, bool DISP>
+__global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIRS>::THREADS)
+    k_stage_flat(const StepArgs a, const float *in, const float *blend) {
+    using L = FlatTile<PAIRS>;
+    __shared__ typename L::Smem sm;
+    float lmax = 0.0f;
+    unsigned nbad = 0;
+    pdl_wait();
+    flat_tile<PAIRS, STAGE, SCHEME, LIM, DISP>(a, in, blend, blockIdx.x * L::X, blockIdx.y * L::ROWS, sm, lmax, nbad);
     if (a.early_launch) pdl_trigger();
     if (a.cfl) block_publish<L::THREADS>(lmax, 0.0f, nbad, a.sc);
 }
@@ -1015,6 +1030,26 @@ __device__ __forceinline__ StepArgs batch_args(const BatchInst &I, int out_role,
     return a;
 }
 
+// Buffer roles and switches of an instance's stage.
+template <int STAGE>
+__device__ __forceinline__ void stage_roles(const BatchInst &I, int &in_role, int &blend_role, int &out_role, int &bc,
+                                            int &cfl) {
+    const bool visc = I.viscous != 0;
+    if (STAGE == 1) {
+        in_role = visc ? ROLE_D : ROLE_N;
+        blend_role = in_role;
+        out_role = ROLE_S;
+        bc = 1;
+        cfl = 0;
+    } else {
+        in_role = ROLE_S;
+        blend_role = visc ? ROLE_D : ROLE_N;
+        out_role = visc ? ROLE_D : ROLE_X;
+        bc = visc ? 0 : 1;
+        cfl = visc ? 0 : 1;
+    }
+}
+
 template <int NT, int K, int STAGE, int SCHEME, int LIM>
 __global__ void __launch_bounds__(NT, 640 / NT) k_stage_batch(const BatchInst *__restrict__ insts,
                                                     const TileDesc *__restrict__ tiles, int ntiles, int rows,
@@ -1036,21 +1071,8 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_stage_batch(const BatchInst *_
     for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
         const TileDesc td = tiles[ti];
         const BatchInst &I = insts[td.inst];
-        const bool visc = I.viscous != 0;
         int in_role, blend_role, out_role, bc, cfl;
-        if (STAGE == 1) {
-            in_role = visc ? ROLE_D : ROLE_N;
-            blend_role = in_role;
-            out_role = ROLE_S;
-            bc = 1;
-            cfl = 0;
-        } else {
-            in_role = ROLE_S;
-            blend_role = visc ? ROLE_D : ROLE_N;
-            out_role = visc ? ROLE_D : ROLE_X;
-            bc = visc ? 0 : 1;
-            cfl = visc ? 0 : 1;
-        }
+        stage_roles<STAGE>(I, in_role, blend_role, out_role, bc, cfl);
         // the tile's arguments live in shared memory, not in registers
         __syncthreads();  // every thread is done with the previous tile's arguments
         if (threadIdx.x == 0) s_args = batch_args(I, out_role, bc, cfl, 1.0f, rows);
@@ -1063,6 +1085,29 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_stage_batch(const BatchInst *_
         if (cfl) block_publish<NT>(lmax, 0.0f, nbad, I.sc);
     }
     if (early_launch) pdl_trigger();
+}
+
+// The batch's stages on flat tiles, one CTA per tile of the list: for batches
+// whose marching tiles would not fill the chip (see the flat stage kernel).
+template <int PAIRS, int STAGE, int SCHEME, int LIM>
+__global__ void __launch_bounds__(FlatTile<PAIRS>::THREADS, 1024 / FlatTile<PAIRS>::THREADS)
+    k_stage_flat_batch(const BatchInst *__restrict__ insts, const TileDesc *__restrict__ tiles, int early_launch) {
+    using L = FlatTile<PAIRS>;
+    __shared__ typename L::Smem sm;
+    __shared__ StepArgs s_args;
+    pdl_wait();
+    const TileDesc td = tiles[blockIdx.x];
+    const BatchInst &I = insts[td.inst];
+    int in_role, blend_role, out_role, bc, cfl;
+    stage_roles<STAGE>(I, in_role, blend_role, out_role, bc, cfl);
+    if (threadIdx.x == 0) s_args = batch_args(I, out_role, bc, cfl, 1.0f, L::ROWS);
+    __syncthreads();
+    float lmax = 0.0f;
+    unsigned nbad = 0;
+    flat_tile<PAIRS, STAGE, SCHEME, LIM, false>(s_args, I.buf[role_buf(I, in_role)], I.buf[role_buf(I, blend_role)],
+                                                td.i0, td.j0, sm, lmax, nbad);
+    if (early_launch) pdl_trigger();
+    if (cfl) block_publish<L::THREADS>(lmax, 0.0f, nbad, I.sc);
 }
 
 template <int NT, int K>
@@ -1548,6 +1593,27 @@ cudaError_t launch_stage_batch(int stage, int scheme, int limiter, const StageTu
     FVM_SB(128, 4) FVM_SB(128, 6) FVM_SB(256, 4) FVM_SB(256, 6)
 #undef FVM_SB
     return cudaErrorInvalidValue;
+}
+
+template <int STAGE>
+static cudaError_t launch_flat_batch_s(int scheme, int lim, const BatchInst *insts, const TileDesc *tiles, int ntiles,
+                                       int early, bool pdl, cudaStream_t st) {
+    using L = FlatTile<kBatchFlatPairs>;
+#define FVM_FB(A, B)                                                                                               \
+    launch_step_kernel(pdl, k_stage_flat_batch<kBatchFlatPairs, STAGE, A, B>, dim3(ntiles), dim3(L::THREADS), 0, st, \
+                       insts, tiles, early)
+    if (scheme == 0 && lim == 0) return FVM_FB(0, 0);
+    if (scheme == 0 && lim == 1) return FVM_FB(0, 1);
+    if (scheme == 1 && lim == 0) return FVM_FB(1, 0);
+    return FVM_FB(1, 1);
+#undef FVM_FB
+}
+
+cudaError_t launch_stage_flat_batch(int stage, int scheme, int limiter, const BatchInst *insts, const TileDesc *tiles,
+                                    int ntiles, int early, bool pdl, cudaStream_t st) {
+    if (ntiles <= 0) return cudaSuccess;
+    return stage == 1 ? launch_flat_batch_s<1>(scheme, limiter, insts, tiles, ntiles, early, pdl, st)
+                      : launch_flat_batch_s<2>(scheme, limiter, insts, tiles, ntiles, early, pdl, st);
 }
 
 template <int NT, int K>

@@ -9,7 +9,7 @@ from helpers import small
 
 pytestmark = pytest.mark.gpu
 
-from fvm_b200 import Solver, abi  # noqa: E402
+from fvm_b200 import Batch, Solver, abi  # noqa: E402
 
 torch = pytest.importorskip("torch")
 
@@ -50,3 +50,24 @@ def test_flat_stage_display_field():
         a = _run(131, 67, workload, abi.FLUX_HLLC, abi.LIMITER_MINMOD, None, True)
         b = _run(131, 67, workload, abi.FLUX_HLLC, abi.LIMITER_MINMOD, (128, 4, 8), True)
         assert np.array_equal(a[4].view(np.uint32), b[4].view(np.uint32))
+
+
+@pytest.mark.parametrize("flux,limiter", [(abi.FLUX_HLLC, abi.LIMITER_VAN_LEER),
+                                          (abi.FLUX_AUSM_PLUS, abi.LIMITER_MINMOD)])
+def test_flat_batch_equals_marching_batch(monkeypatch, flux, limiter):
+    """Uneven sizes, Euler and Navier-Stokes mixed: the default (flat tiles)
+    against a pinned marching shape."""
+    def run():
+        cases = [small(w, nx, ny, flux_scheme=flux, limiter=limiter, mach=2.5)
+                 for w, nx, ny in (("euler_m3_circle", 131, 67), ("ns_karman_re200", 97, 33), ("euler_m3_circle", 37, 19),
+                                   ("ns_karman_re200", 200, 100))]
+        ext = cases[0][1]
+        ext.dt_policy = abi.DT_RECOMPUTE
+        b = Batch(ext)
+        ids = [b.add(p) for p, _ in cases]
+        b.step(7)
+        return [(b.fields(i), b.instance(i).dt, b.instance(i).t_current) for i in ids]
+    a = run()
+    monkeypatch.setenv("FVM_BATCH_TUNE", "128,6,16")
+    for x, y in zip(a, run()):
+        assert np.array_equal(x[0].view(np.uint32), y[0].view(np.uint32)) and x[1:] == y[1:]
