@@ -4,8 +4,9 @@
 // Each instance is a full solve handle (own buffers, geometry, ghost table,
 // device scalars, own CFL time step).  A batched step is six launches for the
 // whole batch (viscous pre-pass, stage 1, ghost pass, stage 2, viscous
-// post-pass, ghost pass + per-instance finalize); each launch is a persistent
-// grid walking a tile list that spans every instance.  Which ping-pong buffer
+// post-pass, ghost pass + per-instance finalize); each launch covers a tile list
+// that spans every instance (flat stage tiles one CTA each, marching tiles in a
+// persistent grid).  Which ping-pong buffer
 // holds U^n is kept per instance on the device, so one captured CUDA graph of
 // a step replays for any number of steps and any mix of instance parities.
 #include <cuda_runtime.h>

@@ -280,9 +280,8 @@ int fvm_set_tune(fvm_handle *h, int nt, int ring, int rows);
 
 /* ------------------------------------------------------------ batches
  * Many independent solves (different grids, Mach numbers, obstacles, Euler
- * or Navier-Stokes) advanced together: each batched step is one persistent
- * launch per stage over a tile list spanning every instance, replayed as one
- * CUDA graph.  Every instance keeps its own time step (the ext's dt policy;
+ * or Navier-Stokes) advanced together: each batched step is one launch per
+ * stage over a tile list spanning every instance, replayed as one CUDA graph.  Every instance keeps its own time step (the ext's dt policy;
  * FVM_DT_RECOMPUTE gives each its own CFL dt).  No reference counterpart. */
 typedef struct fvm_batch fvm_batch;
 int fvm_batch_create(fvm_batch **out, const fvm_ext *ext);
