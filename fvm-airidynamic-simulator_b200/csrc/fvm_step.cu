@@ -549,6 +549,9 @@ struct FlatTile {
 };
 
 // The tile at (i0, j0): everything but the launch order and the reductions.
+// The state is read with ordinary loads: the kernel launches while the ghost
+// pass still writes it, and the read-only path (__ldg) promises nothing for
+// memory written during the kernel's lifetime, pdl_wait or not.
 template <int PAIRS, int STAGE, int SCHEME, int LIM, bool DISP>
 __device__ __forceinline__ void flat_tile(const StepArgs &a, const float *in, const float *blend, int i0, int j0,
                                           typename FlatTile<PAIRS>::Smem &sm, float &lmax, unsigned &nbad) {
@@ -570,9 +573,8 @@ __device__ __forceinline__ void flat_tile(const StepArgs &a, const float *in, co
         for (int h = 0; h < 2; h++) {
             const size_t c = (size_t)clampi(j0 - 2 + 2 * s + h, 0, ny - 1) * g.pitch + col;
             const float *U = in + c;
-            rho[h] = __ldg(U);
-            prim_from_cons(rho[h], __ldg(U + g.plane), __ldg(U + 2 * g.plane), __ldg(U + 3 * g.plane),
-                           __ldg(U + 4 * g.plane), u[h], v[h], p[h], T);
+            rho[h] = U[0];
+            prim_from_cons(rho[h], U[g.plane], U[2 * g.plane], U[3 * g.plane], U[4 * g.plane], u[h], v[h], p[h], T);
             m |= (uint32_t)__ldg(a.mask + c) << (8 * h);
         }
         M[s][x] = (uint16_t)m;
@@ -629,7 +631,7 @@ __device__ __forceinline__ void flat_tile(const StepArgs &a, const float *in, co
         f2 Uc[5], dY[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) {
-            Uc[k] = mk2(__ldg(in + k * g.plane + cell), __ldg(in + k * g.plane + up));
+            Uc[k] = mk2(in[k * g.plane + cell], in[k * g.plane + up]);
             dY[k] = mk2(Fy[k].x - YU[k][p][c], Fy[k].y - Fy[k].x);
         }
         const float4 LA = XA[p][c], RA = XA[p][c + 1], LB = XB[p][c], RB = XB[p][c + 1], LC = XC[p][c],
