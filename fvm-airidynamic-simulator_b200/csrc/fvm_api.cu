@@ -727,10 +727,18 @@ static int error_status(unsigned err) {
 }
 
 // The scalars on the host, once the stream is idle: as the last kernel that
-// changed them wrote them, or else copied.
+// changed them wrote them, or else copied.  Either way the mirror h_sc, which
+// fvm_read_dt reads, holds them too.
 static int sync_scalars(fvm_handle *h) {
     if (h->now_valid) {
         CK(cudaStreamSynchronize(h->stream));
+        const HostScalars &n = *h->h_now;
+        DevScalars &m = *h->h_sc;
+        m.cfl[0] = n.cfl[0];
+        m.cfl[1] = n.cfl[1];
+        m.dt_last = n.dt_last;
+        m.t = n.t;
+        m.err = n.err;
         return FVM_OK;
     }
     CK(cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
