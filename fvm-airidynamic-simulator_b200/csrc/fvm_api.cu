@@ -840,6 +840,7 @@ static int ensure_graphs(fvm_handle *h, int nsteps, cudaGraphExec_t *graphs, uns
         cudaError_t ei = cudaGraphInstantiate(&graphs[par], gr, 0);
         cudaGraphDestroy(gr);
         CK(ei);
+        h->graphs_captured++;
         keys[par] = key;
     }
     return FVM_OK;
@@ -876,6 +877,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
         const int per_step = h->prm.enable_viscosity ? 6 : 4;
         for (; done + 2 <= n; done += 2) {
             CK(cudaGraphLaunch(h->graph[par], h->stream));
+            h->graphs_launched++;
             h->launches += 2 * per_step;
         }
     }
@@ -884,6 +886,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
         const int par = state_parity(h);
         if (int r = ensure_graphs(h, 1, h->graph1, h->graph1_key)) return r;
         CK(cudaGraphLaunch(h->graph1[par], h->stream));
+        h->graphs_launched++;
         h->launches += h->prm.enable_viscosity ? 6 : 4;
         swap_state(h);
         to_host = true;
@@ -1395,6 +1398,13 @@ extern "C" int fvm_debug_ghost_table(fvm_handle *h, int *out, int cap, int *coun
             memcpy(o + 1, &t[k], sizeof(GhostInfo));
         }
     }
+    return FVM_OK;
+}
+
+extern "C" int fvm_debug_graph_count(fvm_handle *h, long long *captured_out, long long *launched_out) {
+    CHECK_HANDLE(h);
+    if (captured_out) *captured_out = h->graphs_captured;
+    if (launched_out) *launched_out = h->graphs_launched;
     return FVM_OK;
 }
 

@@ -59,6 +59,7 @@ struct fvm_handle {
     cudaGraphExec_t graph1[2] = {nullptr, nullptr};
     unsigned long long graph1_key[2] = {0, 0};
     int plain_steps = 0;         // steps launched plainly since the graphs were dropped
+    long long graphs_captured = 0, graphs_launched = 0;  // over the handle's life
     // registered display field (fvm_set_display_field): the last passes of
     // every step write it (destination and kind in the device descriptor
     // d_disp, mirrored in disp / disp_kind); fresh while the state is the one

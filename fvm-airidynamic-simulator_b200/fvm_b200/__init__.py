@@ -39,7 +39,7 @@ EXPORTS = [
     "fvm_state_max_noalloc", "fvm_shedding_stats", "fvm_colormap_to_device", "fvm_colormap_table",
     "fvm_save_checkpoint", "fvm_load_checkpoint", "fvm_checkpoint_info", "fvm_autotune", "fvm_get_tune",
     "fvm_set_tune", "fvm_nonfinite_count", "fvm_debug_stage1", "fvm_debug_ghost_table",
-    "fvm_debug_wait_timeout", "fvm_build_info",
+    "fvm_debug_wait_timeout", "fvm_debug_graph_count", "fvm_build_info",
 ]
 
 
@@ -145,6 +145,7 @@ def load_library(path=None):
     lib.fvm_set_tune.argtypes = [vp, i, i, i]
     lib.fvm_nonfinite_count.argtypes = [vp, C.POINTER(C.c_ulonglong), i]
     lib.fvm_debug_wait_timeout.argtypes = [vp, C.c_longlong]
+    lib.fvm_debug_graph_count.argtypes = [vp, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]
     lib.fvm_debug_ghost_table.argtypes = [vp, vp, i, C.POINTER(i)]
     _lib = lib
     return lib
@@ -357,6 +358,12 @@ class Solver:
         out = np.zeros((max(n.value, 1), 7), np.int32)
         _check(self.lib.fvm_debug_ghost_table(self.h, _p(out), n.value, C.byref(n)))
         return out[:n.value]
+
+    def debug_graph_count(self):
+        """(captured, launched) step graphs of this handle so far."""
+        a, b = C.c_longlong(), C.c_longlong()
+        _check(self.lib.fvm_debug_graph_count(self.h, C.byref(a), C.byref(b)))
+        return a.value, b.value
 
     def autotune(self, steps=6):
         """Pick the fastest launch tuning for this grid class (see fvm_autotune)."""

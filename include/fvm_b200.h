@@ -465,6 +465,10 @@ int fvm_debug_ghost_table(fvm_handle *h, int *out, int cap, int *count_out);
  * the solve's state untouched and usable.  No reference counterpart. */
 int fvm_debug_wait_timeout(fvm_handle *h, long long limit_cycles);
 
+/* Test hook: step graphs captured and launched on this handle since it was
+ * created (either output may be NULL). */
+int fvm_debug_graph_count(fvm_handle *h, long long *captured_out, long long *launched_out);
+
 /* Library build description (arch, flags). */
 const char *fvm_build_info(void);
 
