@@ -198,10 +198,8 @@ static void drop_graphs(fvm_handle *h) {
     for (int k = 0; k < 2; k++) {
         if (h->graph[k]) cudaGraphExecDestroy(h->graph[k]);
         h->graph[k] = nullptr;
-        h->graph_key[k] = 0;
         if (h->graph1[k]) cudaGraphExecDestroy(h->graph1[k]);
         h->graph1[k] = nullptr;
-        h->graph1_key[k] = 0;
     }
 }
 
@@ -696,6 +694,7 @@ static int prepare_dt(fvm_handle *h, fvm_sim_params *p) {
     return FVM_OK;
 }
 
+// What a captured step holds besides the geometry (which drops the graphs by itself).
 static unsigned long long graph_key(fvm_handle *h) {
     unsigned long long k = (unsigned long long)h->prm.enable_viscosity;
     k = k * 31 + h->ext.flux_scheme;
@@ -785,32 +784,29 @@ static int state_parity(fvm_handle *h) {
 constexpr int kGraphAfter = 16, kGraphLongCall = 64;
 
 // Whether the next n steps run as graphs: the one they need exists, or enough
-// steps have run (or very many are asked for) to capture it.  A stream that is itself
-// being captured keeps to the graphs.
+// steps have run (or very many are asked for) to capture it.  A stream that is
+// itself being captured keeps to the graph path, which the runtime refuses there.
 static bool want_graphs(fvm_handle *h, int n) {
-    if (h->plain_steps >= kGraphAfter || n > kGraphLongCall) return true;
     const unsigned long long key = graph_key(h);
+    if (key != h->step_key) {
+        drop_graphs(h);
+        h->step_key = key;
+    }
+    if (h->plain_steps >= kGraphAfter || n > kGraphLongCall) return true;
     const int par = state_parity(h);
-    if (n >= 2 && h->graph[par] && h->graph_key[par] == key) return true;
-    if (n == 1 && h->graph1[par] && h->graph1_key[par] == key) return true;
+    if (n >= 2 ? h->graph[par] != nullptr : h->graph1[par] != nullptr) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(h->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
 }
 
 // Captured graphs of `nsteps` steps (2 or 1) for both buffer parities, built
-// together the first time either is needed (and again after a change of
-// their key), so no later call pays for a capture and an instantiation.  The
-// other parity's graph is captured with the state pointers swapped and
-// restored afterwards; capture launches nothing.
-static int ensure_graphs(fvm_handle *h, int nsteps, cudaGraphExec_t *graphs, unsigned long long *keys) {
+// together the first time either is needed, so no later call pays for a capture
+// and an instantiation.  The other parity's graph is captured with the state
+// pointers swapped and restored afterwards; capture launches nothing.
+static int ensure_graphs(fvm_handle *h, int nsteps, cudaGraphExec_t *graphs) {
     const int cur = state_parity(h);
-    const unsigned long long key = graph_key(h);
     for (int par = 0; par < 2; par++) {
-        if (graphs[par] && keys[par] == key) continue;
-        if (graphs[par]) {
-            cudaGraphExecDestroy(graphs[par]);
-            graphs[par] = nullptr;
-        }
+        if (graphs[par]) continue;
         const bool other = par != cur;
         if (other) swap_state(h);
         cudaGraph_t gr;
@@ -841,7 +837,6 @@ static int ensure_graphs(fvm_handle *h, int nsteps, cudaGraphExec_t *graphs, uns
         cudaGraphDestroy(gr);
         CK(ei);
         h->graphs_captured++;
-        keys[par] = key;
     }
     return FVM_OK;
 }
@@ -873,7 +868,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     bool to_host = false;  // whether the last step queued writes the scalars to the host
     if (use_graph && n >= 2) {
         const int par = state_parity(h);
-        if (int r = ensure_graphs(h, 2, h->graph, h->graph_key)) return r;
+        if (int r = ensure_graphs(h, 2, h->graph)) return r;
         const int per_step = h->prm.enable_viscosity ? 6 : 4;
         for (; done + 2 <= n; done += 2) {
             CK(cudaGraphLaunch(h->graph[par], h->stream));
@@ -884,7 +879,7 @@ extern "C" int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n) {
     if (use_graph && done < n) {
         // one remaining step: a captured single step for this buffer parity
         const int par = state_parity(h);
-        if (int r = ensure_graphs(h, 1, h->graph1, h->graph1_key)) return r;
+        if (int r = ensure_graphs(h, 1, h->graph1)) return r;
         CK(cudaGraphLaunch(h->graph1[par], h->stream));
         h->graphs_launched++;
         h->launches += h->prm.enable_viscosity ? 6 : 4;

@@ -54,10 +54,9 @@ struct fvm_handle {
     // graph replay of two steps, one per buffer parity (which of the two
     // ping-pong buffers currently holds U^n)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    unsigned long long graph_key[2] = {0, 0};
     // graph replay of one step (single-step calls and odd remainders), per parity
     cudaGraphExec_t graph1[2] = {nullptr, nullptr};
-    unsigned long long graph1_key[2] = {0, 0};
+    unsigned long long step_key = 0;  // what the steps since the graphs were dropped depend on (graph_key)
     int plain_steps = 0;         // steps launched plainly since the graphs were dropped
     long long graphs_captured = 0, graphs_launched = 0;  // over the handle's life
     // registered display field (fvm_set_display_field): the last passes of

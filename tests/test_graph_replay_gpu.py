@@ -52,3 +52,29 @@ def test_graph_replay_matches_plain_launches(workload, nx, ny, policy):
         assert n == launches, mode
         assert np.array_equal(got[0].view(np.uint32), ref[0].view(np.uint32)), mode
         assert got[1:] == ref[1:], mode
+
+
+def test_changing_cfl_numbers_never_capture():
+    """A CFL number that changes with every call changes what a captured step
+    holds: such a solve keeps to plain launches, and captures once it stays."""
+    p, e = small("euler_m3_circle", 160, 80)
+    e.dt_policy = abi.DT_RECOMPUTE
+    s = Solver(p, e)
+    q, _ = small("euler_m3_circle", 160, 80)
+    r = Solver(q, e)
+    r.set_kernel_timing(True)
+    for k in range(40):
+        p.cfl = q.cfl = 0.2 + 0.005 * k
+        s.step(1)
+        r.step(1)
+    assert s.debug_graph_count() == (0, 0)
+    s.step(20)
+    s.step(2)
+    r.step(22)
+    assert s.debug_graph_count() == (2, 1)
+    p.cfl = q.cfl = 0.3  # and a change drops them again
+    s.step(3)
+    r.step(3)
+    assert s.debug_graph_count() == (2, 1)
+    assert np.array_equal(s.fields().view(np.uint32), r.fields().view(np.uint32))
+    assert p.dt == q.dt and p.t_current == q.t_current
