@@ -792,7 +792,7 @@ static bool want_graphs(fvm_handle *h, int n) {
         drop_graphs(h);
         h->step_key = key;
     }
-    if (h->plain_steps >= kGraphAfter || n > kGraphLongCall) return true;
+    if (h->plain_steps >= kGraphAfter || n > kGraphLongCall || h->tuning) return true;
     const int par = state_parity(h);
     if (n >= 2 ? h->graph[par] != nullptr : h->graph1[par] != nullptr) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1236,7 +1236,9 @@ extern "C" int fvm_launch_count(fvm_handle *h, long long *count_out) {
 }
 
 // Time each candidate tuning over `steps` steps from a snapshot of the
-// current state (restored after every candidate) and keep the fastest.
+// current state (restored after every candidate) and keep the fastest.  The
+// steps replay graphs, as those of the solve that is tuned will; each
+// candidate's are captured by its warm-up.
 extern "C" int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, float *best_ms_out) {
     CHECK_INIT(h);
     if (!p || steps < 2) return set_err(FVM_ERR_INVALID, "fvm_autotune: need params and steps >= 2");
@@ -1247,6 +1249,7 @@ extern "C" int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, f
     const StageTune before = h->tune;
     const bool timing = h->timing;
     h->timing = false;
+    h->tuning = true;
     fvm_sim_params q = *p;
     StageTune best = before;
     float best_ms = 1e30f;
@@ -1271,7 +1274,7 @@ extern "C" int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, f
         drop_graphs(h);
         if ((rc = build_maps(h)) != FVM_OK) break;
         fvm_sim_params w = q;
-        if ((rc = fvm_steps(h, &w, 3)) != FVM_OK) break;  // warm (captures both graph kinds)
+        if ((rc = fvm_steps(h, &w, 3)) != FVM_OK) break;  // warm: one graph of each kind
         cudaEventRecord(e0, h->stream);
         if ((rc = fvm_steps(h, &w, steps)) != FVM_OK) break;
         cudaEventRecord(e1, h->stream);
@@ -1295,6 +1298,7 @@ extern "C" int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, f
     cudaStreamSynchronize(h->stream);
     cudaFree(snap);
     h->timing = timing;
+    h->tuning = false;
     h->cfl_valid = false;
     h->dt_ready = false;
     h->disp_fresh = false;  // the tuning steps wrote it; the state is restored

@@ -71,6 +71,7 @@ struct fvm_handle {
     float *parity_base = nullptr;  // buffer holding U^n at parity 0
     // measurement
     bool timing = false;
+    bool tuning = false;  // the autotuner's steps: graphs from the first on
     std::vector<TimedLaunch> pending;
     std::vector<cudaEvent_t> event_pool;
     std::map<std::string, std::pair<long long, double>> ktimes;

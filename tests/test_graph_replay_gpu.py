@@ -78,3 +78,21 @@ def test_changing_cfl_numbers_never_capture():
     assert s.debug_graph_count() == (2, 1)
     assert np.array_equal(s.fields().view(np.uint32), r.fields().view(np.uint32))
     assert p.dt == q.dt and p.t_current == q.t_current
+
+
+@pytest.mark.parametrize("steps", [6, 80])
+def test_autotuner_times_graph_replay(steps):
+    """Each candidate captures its graphs while it warms up (3 steps: a
+    two-step and a one-step launch, each kind for both parities) and replays
+    them in the timed steps."""
+    p, e = small("ns_karman_re200", 160, 80)
+    s = Solver(p, e)
+    p.dt = 0.5 * s.compute_dt()
+    U = s.fields()
+    assert s.autotune(steps) > 0
+    captured, launched = s.debug_graph_count()
+    assert captured > 0 and captured % 4 == 0
+    assert launched == captured // 4 * (2 + steps // 2)
+    assert np.array_equal(s.fields().view(np.uint32), U.view(np.uint32))
+    s.step(1)  # the solve itself starts plainly again
+    assert s.debug_graph_count() == (captured, launched)
