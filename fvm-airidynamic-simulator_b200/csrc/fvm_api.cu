@@ -986,23 +986,26 @@ extern "C" int fvm_get_sdf(fvm_handle *h, float *host_sdf) {
     return FVM_OK;
 }
 
-// The five planes of a state (pitched rows, `base` the first) into host arrays of
-// nx*ny floats, queued on the stream: as one copy where the arrays follow each
-// other in memory, as the planes do on the device, else one copy per plane.
+// The five planes of a state (pitched rows, `base` the first) into host arrays
+// of nx*ny floats (null: skipped), queued on the stream.  A copy for each, also
+// where the arrays happen to follow each other: they may be allocations of
+// their own, and the runtime need not accept a copy across page-locked ones.
 int fvm_internal_copy_fields(const GridDesc &g, const float *base, float *const dst[5], cudaStream_t st) {
-    const size_t row = (size_t)g.nx * 4, pitch = (size_t)g.pitch * 4, cells = (size_t)g.nx * g.ny;
-    bool together = dst[0] != nullptr;
-    for (int k = 1; k < 5; k++) together = together && dst[k] == dst[0] + k * cells;
-    if (together) {
-        if (row == pitch)
-            CK(cudaMemcpyAsync(dst[0], base, 5 * cells * 4, cudaMemcpyDeviceToHost, st));
-        else
-            CK(cudaMemcpy2DAsync(dst[0], row, base, pitch, row, (size_t)g.ny * 5, cudaMemcpyDeviceToHost, st));
-        return FVM_OK;
-    }
+    const size_t row = (size_t)g.nx * 4, pitch = (size_t)g.pitch * 4;
     for (int k = 0; k < 5; k++)
         if (dst[k])
             CK(cudaMemcpy2DAsync(dst[k], row, base + (size_t)k * g.plane, pitch, row, g.ny, cudaMemcpyDeviceToHost, st));
+    return FVM_OK;
+}
+
+// The same into one array that holds the planes one after another, as the
+// device does: one copy.
+int fvm_internal_copy_state(const GridDesc &g, const float *base, float *planes, cudaStream_t st) {
+    const size_t row = (size_t)g.nx * 4, pitch = (size_t)g.pitch * 4;
+    if (row == pitch)
+        CK(cudaMemcpyAsync(planes, base, row * g.ny * 5, cudaMemcpyDeviceToHost, st));
+    else
+        CK(cudaMemcpy2DAsync(planes, row, base, pitch, row, (size_t)g.ny * 5, cudaMemcpyDeviceToHost, st));
     return FVM_OK;
 }
 
@@ -1010,6 +1013,14 @@ extern "C" int fvm_read_fields(fvm_handle *h, float *rho, float *rho_u, float *r
     CHECK_INIT(h);
     float *const dst[5] = {rho, rho_u, rho_v, E, rho_e};
     if (int r = fvm_internal_copy_fields(h->g, h->Un, dst, h->stream)) return r;
+    CK(cudaStreamSynchronize(h->stream));
+    return FVM_OK;
+}
+
+extern "C" int fvm_read_state(fvm_handle *h, float *planes) {
+    CHECK_INIT(h);
+    if (!planes) return set_err(FVM_ERR_INVALID, "null buffer");
+    if (int r = fvm_internal_copy_state(h->g, h->Un, planes, h->stream)) return r;
     CK(cudaStreamSynchronize(h->stream));
     return FVM_OK;
 }

@@ -484,17 +484,35 @@ extern "C" int fvm_batch_instance(fvm_batch *b, int id, fvm_sim_params *p_out) {
     return FVM_OK;
 }
 
+// The buffer that holds U^n of an instance, once the batch's stream is idle.
+static int current_state(fvm_batch *b, const fvm_handle *h, const float **src) {
+    BCK(cudaStreamSynchronize(b->stream));
+    unsigned parity = 0;
+    BCK(cudaMemcpy(&parity, &h->sc->parity, sizeof parity, cudaMemcpyDeviceToHost));
+    *src = h->buf[parity ? BUF_X : BUF_N];
+    return FVM_OK;
+}
+
 extern "C" int fvm_batch_read_fields(fvm_batch *b, int id, float *rho, float *rho_u, float *rho_v, float *E,
                                      float *rho_e) {
     CHECK_BATCH(b);
     fvm_handle *h = inst_of(b, id);
     if (!h) return berr(FVM_ERR_INVALID, "unknown instance id");
-    BCK(cudaStreamSynchronize(b->stream));
-    unsigned parity = 0;
-    BCK(cudaMemcpy(&parity, &h->sc->parity, sizeof parity, cudaMemcpyDeviceToHost));
-    const float *src = h->buf[parity ? BUF_X : BUF_N];
+    const float *src = nullptr;
+    if (int r = current_state(b, h, &src)) return r;
     float *const dst[5] = {rho, rho_u, rho_v, E, rho_e};
     if (int r = fvm_internal_copy_fields(h->g, src, dst, b->stream)) return r;
+    BCK(cudaStreamSynchronize(b->stream));
+    return FVM_OK;
+}
+
+extern "C" int fvm_batch_read_state(fvm_batch *b, int id, float *planes) {
+    CHECK_BATCH(b);
+    fvm_handle *h = inst_of(b, id);
+    if (!h || !planes) return berr(FVM_ERR_INVALID, "unknown instance id or null output");
+    const float *src = nullptr;
+    if (int r = current_state(b, h, &src)) return r;
+    if (int r = fvm_internal_copy_state(h->g, src, planes, b->stream)) return r;
     BCK(cudaStreamSynchronize(b->stream));
     return FVM_OK;
 }

@@ -78,9 +78,7 @@ extern "C" int fvm_save_checkpoint(fvm_handle *h, const fvm_sim_params *p, const
     const int nx = h->g.nx, ny = h->g.ny;
     const size_t plane = (size_t)nx * ny;
     std::vector<float> data(plane * 5);
-    if (int r = fvm_read_fields(h, data.data(), data.data() + plane, data.data() + 2 * plane, data.data() + 3 * plane,
-                                data.data() + 4 * plane))
-        return r;
+    if (int r = fvm_read_state(h, data.data())) return r;
     cudaError_t e = cudaMemcpyAsync(h->h_sc, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return ckerr(FVM_ERR_CUDA, cudaGetErrorString(e));

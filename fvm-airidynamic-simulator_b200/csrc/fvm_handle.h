@@ -87,5 +87,6 @@ int fvm_internal_build_maps(fvm_handle *h);
 int fvm_internal_compute_dt(fvm_handle *h, const fvm_sim_params *p, float *dt);
 int fvm_internal_set_error(int code, const char *msg);
 int fvm_internal_copy_fields(const GridDesc &g, const float *base, float *const dst[5], cudaStream_t st);
+int fvm_internal_copy_state(const GridDesc &g, const float *base, float *planes, cudaStream_t st);
 // true when the batch holds a retired instance of this grid size (reused by fvm_batch_add)
 bool fvm_internal_batch_has_parked(fvm_batch *b, int nx, int ny);

@@ -39,6 +39,7 @@ struct Request {
     fvm_sim_params p{};
     int steps = 0;
     float *out[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    float *state = nullptr;  // instead of out: the five planes in one array
     double submit_s = 0, admit_s = 0;
     int id = -1;       // batch instance id once admitted
     int done = 0;      // steps taken
@@ -144,6 +145,7 @@ static fvm_result retire(fvm_server *s, const Request &r, int status) {
     int rc = status;
     if (rc == FVM_OK && (r.out[0] || r.out[1] || r.out[2] || r.out[3] || r.out[4]))
         rc = fvm_batch_read_fields(s->b, r.id, r.out[0], r.out[1], r.out[2], r.out[3], r.out[4]);
+    if (rc == FVM_OK && r.state) rc = fvm_batch_read_state(s->b, r.id, r.state);
     if (rc == FVM_OK) rc = fvm_batch_diagnostics(s->b, r.id, &x.diag);
     fvm_sim_params q;
     if (rc == FVM_OK && (rc = fvm_batch_instance(s->b, r.id, &q)) == FVM_OK) {
@@ -263,16 +265,16 @@ extern "C" int fvm_server_create(fvm_server **out, const fvm_ext *ext, size_t hb
     return FVM_OK;
 }
 
-extern "C" int fvm_server_submit(fvm_server *s, const fvm_sim_params *p, int steps, float *rho, float *rho_u,
-                                 float *rho_v, float *E, float *rho_e, long long *ticket_out) {
+static int submit(fvm_server *s, const fvm_sim_params *p, int steps, float *const out[5], float *state,
+                  long long *ticket_out) {
     if (!s || !p || !ticket_out) return serr(FVM_ERR_INVALID, "null argument");
     if (steps <= 0) return serr(FVM_ERR_INVALID, "fvm_server_submit: steps must be positive");
     if (p->nx <= 0 || p->ny <= 0) return serr(FVM_ERR_INVALID, "fvm_server_submit: nx, ny must be positive");
     Request r;
     r.p = *p;
     r.steps = steps;
-    float *o[5] = {rho, rho_u, rho_v, E, rho_e};
-    for (int k = 0; k < 5; k++) r.out[k] = o[k];
+    for (int k = 0; k < 5; k++) r.out[k] = out[k];
+    r.state = state;
     {
         std::lock_guard<std::mutex> g(s->mu);
         if (s->stop) return serr(FVM_ERR_STATE, "fvm_server_submit: server is stopping");
@@ -284,6 +286,18 @@ extern "C" int fvm_server_submit(fvm_server *s, const fvm_sim_params *p, int ste
     s->cv_work.notify_one();
     *ticket_out = r.ticket;
     return FVM_OK;
+}
+
+extern "C" int fvm_server_submit(fvm_server *s, const fvm_sim_params *p, int steps, float *rho, float *rho_u,
+                                 float *rho_v, float *E, float *rho_e, long long *ticket_out) {
+    float *const out[5] = {rho, rho_u, rho_v, E, rho_e};
+    return submit(s, p, steps, out, nullptr, ticket_out);
+}
+
+extern "C" int fvm_server_submit_state(fvm_server *s, const fvm_sim_params *p, int steps, float *planes,
+                                       long long *ticket_out) {
+    float *const none[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    return submit(s, p, steps, none, planes, ticket_out);
 }
 
 extern "C" int fvm_server_poll(fvm_server *s, fvm_result *out, int cap, int *n_out) {

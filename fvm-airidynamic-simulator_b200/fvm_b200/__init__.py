@@ -24,7 +24,7 @@ EXPORTS = [
     "fvm_last_error", "fvm_params_compute_derived", "fvm_params_default", "fvm_ext_default",
     "fvm_create", "fvm_destroy", "fvm_set_stream", "fvm_initialize", "fvm_resize", "fvm_reset",
     "fvm_update_obstacle", "fvm_set_ext", "fvm_step", "fvm_steps", "fvm_compute_dt", "fvm_queue_dt",
-    "fvm_read_dt", "fvm_synchronize", "fvm_get_cell_types", "fvm_get_sdf", "fvm_read_fields",
+    "fvm_read_dt", "fvm_synchronize", "fvm_get_cell_types", "fvm_get_sdf", "fvm_read_fields", "fvm_read_state",
     "fvm_read_region", "fvm_read_region_geometry",
     "fvm_write_fields", "fvm_read_primitives", "fvm_field_to_device", "fvm_set_display_field",
     "fvm_cell_types_to_device",
@@ -32,9 +32,9 @@ EXPORTS = [
     "fvm_diagnostics", "fvm_shock_standoff", "fvm_set_kernel_timing", "fvm_kernel_times",
     "fvm_launch_count", "fvm_batch_create", "fvm_batch_destroy", "fvm_batch_set_stream", "fvm_batch_add",
     "fvm_batch_remove", "fvm_batch_count", "fvm_batch_step", "fvm_batch_synchronize", "fvm_batch_instance",
-    "fvm_batch_read_fields", "fvm_batch_diagnostics", "fvm_batch_nonfinite_count", "fvm_batch_memory_usage",
+    "fvm_batch_read_fields", "fvm_batch_read_state", "fvm_batch_diagnostics", "fvm_batch_nonfinite_count", "fvm_batch_memory_usage",
     "fvm_batch_launch_count",
-    "fvm_batch_instance_bytes", "fvm_batch_retire", "fvm_batch_trim", "fvm_server_create", "fvm_server_submit",
+    "fvm_batch_instance_bytes", "fvm_batch_retire", "fvm_batch_trim", "fvm_server_create", "fvm_server_submit", "fvm_server_submit_state",
     "fvm_server_poll", "fvm_server_wait", "fvm_server_drain", "fvm_server_get_stats", "fvm_server_destroy",
     "fvm_state_max_noalloc", "fvm_shedding_stats", "fvm_colormap_to_device", "fvm_colormap_table",
     "fvm_save_checkpoint", "fvm_load_checkpoint", "fvm_checkpoint_info", "fvm_autotune", "fvm_get_tune",
@@ -89,6 +89,7 @@ def load_library(path=None):
     lib.fvm_get_cell_types.argtypes = [vp, vp]
     lib.fvm_get_sdf.argtypes = [vp, vp]
     lib.fvm_read_fields.argtypes = [vp] + [vp] * 5
+    lib.fvm_read_state.argtypes = [vp, vp]
     lib.fvm_read_region.argtypes = [vp, i, i, i, i] + [vp] * 5
     lib.fvm_read_region_geometry.argtypes = [vp, i, i, i, i, vp, vp]
     lib.fvm_write_fields.argtypes = [vp] + [vp] * 5
@@ -123,6 +124,7 @@ def load_library(path=None):
     lib.fvm_batch_synchronize.argtypes = [vp]
     lib.fvm_batch_instance.argtypes = [vp, i, Pp]
     lib.fvm_batch_read_fields.argtypes = [vp, i] + [vp] * 5
+    lib.fvm_batch_read_state.argtypes = [vp, i, vp]
     lib.fvm_batch_diagnostics.argtypes = [vp, i, C.POINTER(Diag)]
     lib.fvm_batch_nonfinite_count.argtypes = [vp, i, C.POINTER(C.c_ulonglong)]
     lib.fvm_batch_memory_usage.argtypes = [vp, C.POINTER(sz)]
@@ -136,6 +138,7 @@ def load_library(path=None):
     lib.fvm_batch_trim.argtypes = [vp, sz, C.POINTER(sz)]
     lib.fvm_server_create.argtypes = [C.POINTER(vp), C.POINTER(Ext), sz, i, i]
     lib.fvm_server_submit.argtypes = [vp, Pp, i, vp, vp, vp, vp, vp, C.POINTER(C.c_longlong)]
+    lib.fvm_server_submit_state.argtypes = [vp, Pp, i, vp, C.POINTER(C.c_longlong)]
     lib.fvm_server_poll.argtypes = [vp, C.POINTER(Result), i, C.POINTER(i)]
     lib.fvm_server_wait.argtypes = [vp, C.c_longlong, C.c_double, C.POINTER(Result)]
     lib.fvm_server_drain.argtypes = [vp, C.c_double]
@@ -161,8 +164,8 @@ def _p(a):
 
 
 def _planes(k, *shape):
-    """(array, pointers): k float32 planes of `shape` in one array, which the
-    library then fills with one copy instead of k arrays to be stacked after."""
+    """(array, pointers): k float32 planes of `shape` in one array, filled in
+    place instead of k arrays to be stacked after."""
     a = np.empty((k,) + shape, np.float32)
     return a, [C.c_void_p(a.ctypes.data + i * a.strides[0]) for i in range(k)]
 
@@ -240,8 +243,8 @@ class Solver:
 
     # readback --------------------------------------------------------------
     def fields(self):
-        out, ptrs = _planes(5, *self.shape)
-        _check(self.lib.fvm_read_fields(self.h, *ptrs))
+        out = np.empty((5,) + self.shape, np.float32)
+        _check(self.lib.fvm_read_state(self.h, _p(out)))
         return out
 
     def read_region(self, i0, j0, w, h):
@@ -455,8 +458,8 @@ class Batch:
         return p
 
     def fields(self, id_):
-        out, ptrs = _planes(5, *self.shapes[id_])
-        _check(self.lib.fvm_batch_read_fields(self.h, int(id_), *ptrs))
+        out = np.empty((5,) + self.shapes[id_], np.float32)
+        _check(self.lib.fvm_batch_read_state(self.h, int(id_), _p(out)))
         return out
 
     def diagnostics(self, id_):
@@ -511,18 +514,14 @@ class Server:
     def submit(self, params, steps, keep_fields=True):
         """Queue a solve of `steps` steps; returns its ticket."""
         t = C.c_longlong()
-        if keep_fields:
-            arrs, ptrs = _planes(5, params.ny, params.nx)
-        else:
-            arrs, ptrs = None, [None] * 5
-        _check(self.lib.fvm_server_submit(self.h, C.byref(params), int(steps), *ptrs, C.byref(t)))
-        self.outputs[t.value] = arrs
+        out = np.empty((5, params.ny, params.nx), np.float32) if keep_fields else None
+        _check(self.lib.fvm_server_submit_state(self.h, C.byref(params), int(steps), _p(out), C.byref(t)))
+        self.outputs[t.value] = out
         return t.value
 
     def _collect(self, r):
-        arrs = self.outputs.pop(r.ticket, None)
-        fields = arrs if arrs is not None and r.status == 0 else None
-        return r, fields
+        out = self.outputs.pop(r.ticket, None)
+        return r, out if r.status == 0 else None
 
     def wait(self, ticket, timeout_s=-1.0):
         """(Result, fields or None) of one request."""

@@ -170,6 +170,9 @@ int fvm_get_sdf(fvm_handle *h, float *host_sdf);
  * its private d_rho_ ... d_rho_e_, src/include/solver.cuh:92-96).  Any pointer
  * may be NULL to skip that field.  fvm_write_fields recomputes primitives. */
 int fvm_read_fields(fvm_handle *h, float *rho, float *rho_u, float *rho_v, float *E, float *rho_e);
+/* The same fields into one array of 5*nx*ny floats, plane after plane: one
+ * copy instead of five. */
+int fvm_read_state(fvm_handle *h, float *planes);
 /* The [i0, i0+w) x [j0, j0+hgt) window of the conserved fields into host
  * arrays of w*hgt floats (row-major; NULL skips a field), for probes and
  * windows of grids too large to copy whole.  No reference counterpart. */
@@ -297,6 +300,8 @@ int fvm_batch_synchronize(fvm_batch *b);
 /* Instance parameters with its t_current, step and last dt. */
 int fvm_batch_instance(fvm_batch *b, int id, fvm_sim_params *p_out);
 int fvm_batch_read_fields(fvm_batch *b, int id, float *rho, float *rho_u, float *rho_v, float *E, float *rho_e);
+/* The same into one array of 5*nx*ny floats (see fvm_read_state). */
+int fvm_batch_read_state(fvm_batch *b, int id, float *planes);
 int fvm_batch_diagnostics(fvm_batch *b, int id, fvm_diag *out);
 /* The instance's non-finite (cell, step) count (fvm_nonfinite_count) since it
  * was added or reset for its current solve.  No reference counterpart. */
@@ -356,6 +361,9 @@ int fvm_server_create(fvm_server **out, const fvm_ext *ext, size_t hbm_budget_by
  * they must stay valid until the result is collected. */
 int fvm_server_submit(fvm_server *s, const fvm_sim_params *p, int steps, float *rho, float *rho_u, float *rho_v,
                       float *E, float *rho_e, long long *ticket_out);
+/* The same with the final state in one array of 5*nx*ny floats (see
+ * fvm_read_state; NULL: not wanted). */
+int fvm_server_submit_state(fvm_server *s, const fvm_sim_params *p, int steps, float *planes, long long *ticket_out);
 /* Collect up to cap finished results (completion order); *n_out receives how many. */
 int fvm_server_poll(fvm_server *s, fvm_result *out, int cap, int *n_out);
 /* Wait for one request's result (timeout_s < 0: no limit); FVM_ERR_TIMEOUT if it did not finish in time. */
