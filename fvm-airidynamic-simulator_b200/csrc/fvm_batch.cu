@@ -82,21 +82,27 @@ static int batch_rows(const fvm_batch *b) {
     return 4;
 }
 
-static long long batch_cells(const fvm_batch *b) {
-    long long n = 0;
+// Whether a batch's stages run on flat tiles.  The persistent marching stages
+// keep their arguments in shared memory and run 5 CTAs per SM with spills, so
+// batches of few cells are better flat beyond a single solve's limit; with more
+// cells the flat tiles' halo costs more than that, except where narrow grids
+// fill the marching strips (`strip` columns) badly and idle lanes cost as much.
+// Measured flat / marching step times, 2M, 4M, 8M, 12-16M cells of one size:
+// strips full (620x310 to 4096x2048, 3 % idle at most): Euler 0.90-0.95,
+// 0.94-1.01, 0.96-1.06, 0.96-1.08; Navier-Stokes 0.94-0.95, 0.98-1.01,
+// 0.98-1.05, 1.03-1.06.  1024x512 (9 % idle): Euler 0.87, 0.97, 0.98, 0.96,
+// Navier-Stokes 0.91, 0.98, 0.99, 1.01; 512x256 (21 %): 0.80, 0.83, 0.85,
+// 0.86-0.93; 256x128 (45 %): 0.85, 0.85, 0.90, 0.90.
+static bool batch_flat(const fvm_batch *b, int strip) {
+    constexpr long long kFull = 3500000, kIdle = 16000000;
+    long long cells = 0, covered = 0;
     for (const fvm_handle *h : b->slots)
-        if (h) n += (long long)h->g.nx * h->g.ny;
-    return n;
+        if (h) {
+            cells += (long long)h->g.nx * h->g.ny;
+            covered += (long long)((h->g.nx + strip - 1) / strip) * strip * h->g.ny;
+        }
+    return cells <= kFull || (cells <= kIdle && covered * 20 >= cells * 21);
 }
-
-// Cells up to which a batch's stages run on flat tiles.  The limit is higher than
-// a single solve's: the persistent marching stages keep their arguments in
-// shared memory and run 5 CTAs per SM with spills, and the narrow grids of a
-// batch fill their 124-column strips badly.  Measured steps, marching -> flat:
-// 16 solves 0.3M cells 81.9 -> 65.2 us, 1.5M 178.9 -> 151.2, 64 solves 9.1M
-// 724 -> 698, 11.8M 920 -> 884, 128 solves 22.7M 1617 -> 1645, 256 solves 43.9M
-// 3208 -> 3202 us.
-constexpr long long kBatchFlatCells = 16000000;
 
 // Rebuild the device descriptors and tile lists after the set of instances changed.
 static int rebuild(fvm_batch *b) {
@@ -105,7 +111,7 @@ static int rebuild(fvm_batch *b) {
     std::vector<GhostChunk> chunks;
     if (!b->tune_fixed) b->tune.rows = batch_rows(b);
     const int W = stage_cols_per_cta(b->tune), rows = b->tune.rows;
-    b->flat = !b->tune_fixed && batch_cells(b) <= kBatchFlatCells;
+    b->flat = !b->tune_fixed && batch_flat(b, W);
     for (size_t id = 0; id < b->slots.size(); id++) {
         fvm_handle *h = b->slots[id];
         if (!h) continue;
@@ -551,6 +557,15 @@ extern "C" int fvm_batch_memory_usage(fvm_batch *b, size_t *bytes) {
         t += x;
     }
     *bytes = t;
+    return FVM_OK;
+}
+
+extern "C" int fvm_debug_batch_flat(fvm_batch *b, int *flat_out) {
+    CHECK_BATCH(b);
+    if (!flat_out) return berr(FVM_ERR_INVALID, "null output");
+    if (b->dirty)
+        if (int r = rebuild(b)) return r;
+    *flat_out = b->flat ? 1 : 0;
     return FVM_OK;
 }
 

@@ -39,7 +39,8 @@ EXPORTS = [
     "fvm_state_max_noalloc", "fvm_shedding_stats", "fvm_colormap_to_device", "fvm_colormap_table",
     "fvm_save_checkpoint", "fvm_load_checkpoint", "fvm_checkpoint_info", "fvm_autotune", "fvm_get_tune",
     "fvm_set_tune", "fvm_nonfinite_count", "fvm_debug_stage1", "fvm_debug_ghost_table",
-    "fvm_debug_wait_timeout", "fvm_debug_graph_count", "fvm_build_info",
+    "fvm_debug_wait_timeout", "fvm_debug_graph_count", "fvm_debug_batch_flat",
+    "fvm_build_info",
 ]
 
 
@@ -149,6 +150,7 @@ def load_library(path=None):
     lib.fvm_nonfinite_count.argtypes = [vp, C.POINTER(C.c_ulonglong), i]
     lib.fvm_debug_wait_timeout.argtypes = [vp, C.c_longlong]
     lib.fvm_debug_graph_count.argtypes = [vp, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]
+    lib.fvm_debug_batch_flat.argtypes = [vp, C.POINTER(i)]
     lib.fvm_debug_ghost_table.argtypes = [vp, vp, i, C.POINTER(i)]
     _lib = lib
     return lib
@@ -472,6 +474,12 @@ class Batch:
         v = C.c_ulonglong()
         _check(self.lib.fvm_batch_nonfinite_count(self.h, int(id_), C.byref(v)))
         return v.value
+
+    def debug_flat(self):
+        """Whether the stages run on the flat kernel (else they march)."""
+        v = C.c_int()
+        _check(self.lib.fvm_debug_batch_flat(self.h, C.byref(v)))
+        return bool(v.value)
 
     def memory_usage(self):
         v = C.c_size_t()

@@ -477,6 +477,9 @@ int fvm_debug_wait_timeout(fvm_handle *h, long long limit_cycles);
  * created (either output may be NULL). */
 int fvm_debug_graph_count(fvm_handle *h, long long *captured_out, long long *launched_out);
 
+/* Test hook: whether the batch's stages run on the flat kernel (1) or march (0). */
+int fvm_debug_batch_flat(fvm_batch *b, int *flat_out);
+
 /* Library build description (arch, flags). */
 const char *fvm_build_info(void);
 
