@@ -202,18 +202,26 @@ __global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__res
 }
 
 // cellTypeToFloatKernel (src/solver.cu:3444-3450); both arrays are dense, four
-// cells per thread where the destination is 16-byte aligned (VEC).
+// cells per thread: side by side where the destination is 16-byte aligned
+// (VEC), else 256 apart, so that a warp's scalar stores are consecutive.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_ct_to_float(long long n, const uint8_t *__restrict__ ct,
                                                      float *__restrict__ dst) {
-    const long long e = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
-    if (VEC && e + 4 <= n) {
-        const uchar4 c = *reinterpret_cast<const uchar4 *>(ct + e);
-        *reinterpret_cast<float4 *>(dst + e) =
-            make_float4(static_cast<float>(c.x), static_cast<float>(c.y), static_cast<float>(c.z), static_cast<float>(c.w));
-        return;
+    if (VEC) {
+        const long long e = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+        if (e + 4 <= n) {
+            const uchar4 c = *reinterpret_cast<const uchar4 *>(ct + e);
+            *reinterpret_cast<float4 *>(dst + e) = make_float4(static_cast<float>(c.x), static_cast<float>(c.y),
+                                                               static_cast<float>(c.z), static_cast<float>(c.w));
+            return;
+        }
+        for (long long k = e; k < n; k++) dst[k] = static_cast<float>(ct[k]);
+    } else {
+        const long long e = (long long)blockIdx.x * 1024 + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (e + 256 * k < n) dst[e + 256 * k] = static_cast<float>(ct[e + 256 * k]);
     }
-    for (long long k = e; k < e + 4 && k < n; k++) dst[k] = static_cast<float>(ct[k]);
 }
 
 // WHAT = 0: max temperature of the primitives (getMaxTemperature,
