@@ -202,17 +202,24 @@ def serving_requests(n, lam, seed=SERVE_SEED):
     return out
 
 
+# plain steps after which a solver captures its step graphs (fvm_steps)
+GRAPH_AFTER = 16
+
+
 def _events(torch):
     return torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
 
 
 def solo_rate(torch, fvm_b200, p, ext, stream, steps):
-    """Device time of `steps` single-solve steps (graphs warmed for both parities)."""
+    """Device time of `steps` single-solve steps, which replay step graphs:
+    the solver captures them after 16 plain steps, the two-step kind in the
+    second call and the one-step kind in the third."""
     s = fvm_b200.Solver(abi.SimParams.from_buffer_copy(p), ext)
     s.set_stream(stream.cuda_stream)
     with torch.cuda.stream(stream):
-        s.step(3)
-        s.step(3)
+        s.step(GRAPH_AFTER)
+        s.step(2)
+        s.step(1)
         ev0, ev1 = _events(torch)
         ev0.record(stream)
         s.step(steps)
@@ -438,6 +445,7 @@ def grid_scaling(torch, fvm_b200, nx=4096, ny=2048, steps=20, settle=20):
     with torch.cuda.stream(stream):
         s.step(settle)
         s.autotune(steps=4)
+        s.step(GRAPH_AFTER)
         s.step(5)
         ev0, ev1 = _events(torch)
         ev0.record(stream)
@@ -704,9 +712,11 @@ def main():
         s.step(args.settle)
         if not args.no_autotune:
             s.autotune(steps=4)  # launch shape for this grid class (untimed)
-        # W warm-up steps as W-1 and 1: the first call captures the two-step
-        # graphs, the second the one-step graphs (both buffer parities each),
-        # so the timed steps replay graphs and capture none
+        # the plain steps before a solver's first capture belong to the
+        # settling; then W warm-up steps as W-1 and 1: the first call captures
+        # the two-step graphs, the second the one-step graphs (both buffer
+        # parities each), so the timed steps replay graphs and capture none
+        s.step(GRAPH_AFTER)
         s.step(max(args.warmup - 1, 2))
         s.step(1)
         torch.cuda.synchronize()
@@ -788,7 +798,8 @@ def main():
             fvm_b200._check(lib.fvm_set_display_field(s.h, abi.FIELD_MACH,
                                                       C.c_void_p(field.data_ptr() if display else None)))
             fvm_b200._check(lib.fvm_compute_dt(s.h, C.byref(s.params), C.byref(dt_c)))
-            for _ in range(args.warmup):
+            # past the plain steps and the capture of the one-step graphs
+            for _ in range(max(args.warmup, GRAPH_AFTER + 2)):
                 frame()
             barrier(dist)
             torch.cuda.synchronize()
@@ -804,7 +815,10 @@ def main():
         app_max, app_stats_reads = frame_loop(True)
         fvm_b200._check(lib.fvm_set_display_field(s.h, abi.FIELD_MACH, None))
         s.set_ext(ext)
-        s.step(3)  # captures the step graphs again (a new policy drops them)
+        # a new policy drops the step graphs: plain steps, then a call that
+        # captures both kinds again
+        s.step(GRAPH_AFTER)
+        s.step(3)
         torch.cuda.synchronize()
 
         # ---- end to end with the whole state through host memory: upload
