@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__res
             if ((m4 >> (8 * k)) & MB_WALL) {
                 r = gr = b = 0.3f;
             } else {
-                const float s = fminf(fmaxf((in.value(k) - lo) / (hi - lo + 0.0001f), 0.0f), 1.0f);
+                // the value rounded before lo comes off: fused with its last
+                // product in some variants, bytes depended on the variant
+                const float s = fminf(fmaxf(__fsub_rn(in.value(k), lo) / (hi - lo + 0.0001f), 0.0f), 1.0f);
                 const float u = s * 256.0f - 0.5f;
                 const float fl = floorf(u);
                 const float w = u - fl;
