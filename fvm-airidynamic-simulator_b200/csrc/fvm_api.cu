@@ -264,7 +264,8 @@ static int march_rows(int nx, int ny, int slots) {
 // through its row pairs one after another (2 us each, the latency of one
 // pair's dependent arithmetic) and taller tiles mean fewer CTAs, while the flat
 // kernel has a thread for every face at once; above, the flat kernel's
-// two-cell halo (1.6 times the cells of a 32x14 tile) costs more than that.
+// two-cell halo (1.45 times the cells of a 32x14 tile, 1.88 of a 32x6 one) costs
+// more than that.
 // Measured Euler steps, marching (best rows) -> flat, us: 256x128 22.6 -> 16.4,
 // 512x256 27.3 -> 20.6, 1024x512 49.2 -> 40.0, 1501x777 77.3 -> 72.7, 1800x900
 // 96.6 -> 98.8, 2048x1024 116.9 -> 123.7.  Tiles of 32x14 cells, or of 32x6
@@ -994,7 +995,8 @@ int fvm_internal_copy_fields(const GridDesc &g, const float *base, float *const 
     const size_t row = (size_t)g.nx * 4, pitch = (size_t)g.pitch * 4;
     for (int k = 0; k < 5; k++)
         if (dst[k])
-            CK(cudaMemcpy2DAsync(dst[k], row, base + (size_t)k * g.plane, pitch, row, g.ny, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpy2DAsync(dst[k], row, base + (size_t)k * g.plane, pitch, row, g.ny, cudaMemcpyDeviceToHost,
+                                 st));
     return FVM_OK;
 }
 
@@ -1420,5 +1422,5 @@ extern "C" int fvm_debug_graph_count(fvm_handle *h, long long *captured_out, lon
 
 extern "C" const char *fvm_build_info(void) {
     return "fvm_b200: sm_100a, nvcc " FVM_STR(__CUDACC_VER_MAJOR__) "." FVM_STR(__CUDACC_VER_MINOR__)
-           ", --use_fast_math, marching TMA stage kernels";
+           ", --use_fast_math, marching TMA and flat stage kernels";
 }

@@ -128,7 +128,7 @@ __device__ const ColormapLUT kColorTables[5] = {colormap_lut(0), colormap_lut(1)
 // lookup is two vector loads; indexed in the kernel's parameters (constant
 // memory), lanes with different entries were served one after the other.
 // Mach -> RGBA8 at 8192x4096: 214 us indexed in constant memory, 112 us here
-// (21 B per cell, 6.3 TB/s); Mach -> RGBA float at 5000x2500 94 -> 71.
+// (21 B per cell, 6.3-6.5 TB/s); Mach -> RGBA float at 5000x2500 94 -> 71.
 template <int KIND, int FMT, bool GROUP>
 __global__ void __launch_bounds__(256) k_colormap(GridDesc g, const float *__restrict__ U,
                                                   const uint8_t *__restrict__ mask, int colormap, float lo,
@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(256) k_ct_to_float(long long n, const uint8_t 
 // src/solver.cu:2835-2867); WHAT = 1: max local Mach (computeMachNumberKernel,
 // src/solver.cu:2782-2794).  The last block writes the maximum to `out` in
 // pinned host memory and leaves the scratch {maximum, counter} zero for the
-// next call: no memset before and no copy after.  2048x1024: 12.4 us one cell at a time,
-// 10.0 us here.
+// next call: no memset before and no copy after.  2048x1024: 12.4 us one cell
+// at a time, 10.0 us here.
 template <int WHAT>
 __global__ void __launch_bounds__(256, 6) k_max_reduce(GridDesc g, const float *__restrict__ U, float *scratch,
                                                     float *out) {

@@ -355,8 +355,8 @@ __device__ __forceinline__ void stress_heat_mu(float mu_val, float uC, float vC,
 // itself and fx (fy) = 1/dx (1/dy); at a right (top) edge the east (north)
 // one, likewise; in the interior the neighbours and 1/(2dx), 1/(2dy): every
 // difference is the one stress_heat_mu takes, with identical operations),
-// plus what the divergence of the viscous update needs from this cell: the work terms u tau_xx + v tau_xy and u tau_xy + v tau_yy, and
-// the dissipation Phi = tau_xx du/dx + tau_yy dv/dy + tau_xy (du/dy + dv/dx)
+// plus what the divergence of the viscous update needs from this cell: the work
+// terms u tau_xx + v tau_xy and u tau_xy + v tau_yy, and the dissipation Phi = tau_xx du/dx + tau_yy dv/dy + tau_xy (du/dy + dv/dx)
 // (src/solver.cu:2437-2510).  out = {txx, tyy, txy, qx, qy, wx, wy, phi}.
 // In the interior (the only cells the update changes) the velocity
 // gradients are the central differences the reference's update uses.

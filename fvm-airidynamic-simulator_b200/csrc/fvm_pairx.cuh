@@ -17,8 +17,9 @@
 // (src/solver.cu:1502-1598 / :1601-1682) with its HLLC (:1112-1223 /
 // :1315-1430) or AUSM+, the update that of updateKernel (:1736-1875), with
 // explicit fused multiply-adds and one approximate reciprocal per shared
-// divisor, so results can differ from the reference's in the last bits.  The x-face ring stores each row pair interleaved as well, so the
-// update's flux differences come out of vector loads as register pairs.
+// divisor, so results can differ from the reference's in the last bits.  The
+// x-face ring stores each row pair interleaved as well, so the update's flux
+// differences come out of vector loads as register pairs.
 #pragma once
 #include "fvm_math.cuh"
 
@@ -127,7 +128,8 @@ __device__ __forceinline__ void hllc_pair(const f2 &rL, const f2 &nL, const f2 &
     const f2 ds = p_sub(mL, mR);
     const f2 sds = mk2(fminf(ds.x, -1e-10f), fminf(ds.y, -1e-10f));
     const f2 Ss = p_div(p_sub(p_fma(mL, nL, p_sub(pR, pL)), p_mul(mR, nR)), sds);
-    // upwind side K of the wave fan (see hllc_flux)
+    // upwind side K of the wave fan: the left state if all waves or the contact
+    // move right, else the right one (the reference branches four ways)
     const bool supL0 = SL.x >= 0.0f, supL1 = SL.y >= 0.0f;
     const bool supR0 = !supL0 && SR.x <= 0.0f, supR1 = !supL1 && SR.y <= 0.0f;
     const bool useL0 = supL0 || (!supR0 && Ss.x >= 0.0f), useL1 = supL1 || (!supR1 && Ss.y >= 0.0f);
@@ -198,7 +200,8 @@ __device__ __forceinline__ void ausm_plus_pair(const f2 &rL, const f2 &nL, const
     const f2 al = p_add(cl, one), bl = p_fma(cl, cl, splat(-1.0f));
     const f2 al4 = p_mul(quarter, al);
     const f2 mp = p_add(p_fma(al4, al, p_mul(p_mul(eighth, bl), bl)), p_max(p_sub(ML, one), 0.0f));
-    const f2 pp = p_fma(p_mul(al4, al), p_fma(cl, splat(-1.0f), splat(2.0f)), p_mul(p_mul(p_mul(splat(0.1875f), cl), bl), bl));
+    const f2 pp = p_fma(p_mul(al4, al), p_fma(cl, splat(-1.0f), splat(2.0f)),
+                        p_mul(p_mul(p_mul(splat(0.1875f), cl), bl), bl));
     // M- = -(M-1)^2/4 - (M^2-1)^2/8, P- = (M-1)^2 (2+M)/4 - 3/16 M (M^2-1)^2
     const f2 ar = p_sub(cr, one), br = p_fma(cr, cr, splat(-1.0f));
     const f2 ar4 = p_mul(quarter, ar);

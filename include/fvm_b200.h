@@ -148,7 +148,8 @@ int fvm_step(fvm_handle *h, fvm_sim_params *p);
  * for fvm_step) once 16 steps have run, or when more than 64 are asked for;
  * until then they are launched plainly.  The first call that needs a graph kind captures
  * it for both ping-pong buffer parities; a change of launch shape, dt policy,
- * CFL numbers, viscosity switches, geometry or stream drops the graphs. */
+ * CFL numbers, viscosity switches, geometry or stream drops the graphs and the
+ * count starts again. */
 int fvm_steps(fvm_handle *h, fvm_sim_params *p, int n);
 /* CFDSolver::computeStableTimeStep (src/solver.cu:3273-3278). */
 int fvm_compute_dt(fvm_handle *h, const fvm_sim_params *p, float *dt_out);
@@ -205,7 +206,8 @@ int fvm_field_to_device(fvm_handle *h, int kind, float *dev_dst);
  * left (writing fields, reset, obstacle updates, checkpoint loads and the
  * autotuner make it launch again).  dev_dst must stay valid while it is
  * registered; dev_dst == NULL unregisters, and so do fvm_initialize and
- * fvm_resize.  Changing the registration re-captures the step graphs. */
+ * fvm_resize.  Registering a first buffer and unregistering drop the step
+ * graphs; another buffer or kind does not. */
 int fvm_set_display_field(fvm_handle *h, int kind, float *dev_dst);
 /* CFDSolver::convertCellTypesToDevice (src/solver.cu:3452-3459). */
 int fvm_cell_types_to_device(fvm_handle *h, float *dev_dst);
@@ -265,17 +267,19 @@ int fvm_kernel_times(fvm_handle *h, fvm_kernel_time *out, int cap, int *count_ou
 
 /* Autotuner: times the default launch shape (on small grids: stages on the
  * flat kernel) and every candidate launch tuning of the marching step kernels
- * (threads per CTA 128/256, TMA ring depth 4/6 rows, rows per CTA 4..256) over `steps` steps of this solve, restoring the state after each,
- * keeps the fastest for this handle and caches it for the grid class (grid
- * size, viscous flag, flux scheme, limiter) for later handles in the process.
+ * (threads per CTA 128/256, TMA ring depth 4/6 rows, rows per CTA 4..256) on
+ * graph replay over `steps` steps of this solve, restoring the state after
+ * each, keeps the fastest for this handle and caches it for the grid class
+ * (grid size, viscous flag, flux scheme, limiter) for later handles in the
+ * process.
  * *best_ms_out receives the winner's time per step. */
 int fvm_autotune(fvm_handle *h, const fvm_sim_params *p, int steps, float *best_ms_out);
 /* The launch tuning of the marching kernels in use (by default small grids run
  * their stages on the flat kernel, which this tuning does not describe). */
 int fvm_get_tune(fvm_handle *h, int *nt, int *ring, int *rows);
 /* Pin a launch tuning (e.g. one an earlier fvm_autotune chose) of the marching
- * kernels, which then run on every grid size: threads per CTA 128 or 256, ring depth 4 or 6 rows, an even number of rows per CTA in
- * 4..65536.  Results are bitwise the same under every allowed tuning; only the
+ * kernels, which then run on every grid size: threads per CTA 128 or 256, ring
+ * depth 4 or 6 rows, an even number of rows per CTA in 4..65536.  Results are bitwise the same under every allowed tuning; only the
  * speed differs.  (Tiles start on even rows, so a row always takes the same
  * place in the row pair the kernels evaluate together; the two places are
  * separately compiled code and may round differently in the last bit.) */
@@ -284,7 +288,8 @@ int fvm_set_tune(fvm_handle *h, int nt, int ring, int rows);
 /* ------------------------------------------------------------ batches
  * Many independent solves (different grids, Mach numbers, obstacles, Euler
  * or Navier-Stokes) advanced together: each batched step is one launch per
- * stage over a tile list spanning every instance, replayed as one CUDA graph.  Every instance keeps its own time step (the ext's dt policy;
+ * stage over a tile list spanning every instance, replayed as one CUDA graph.
+ * Every instance keeps its own time step (the ext's dt policy;
  * FVM_DT_RECOMPUTE gives each its own CFL dt).  No reference counterpart. */
 typedef struct fvm_batch fvm_batch;
 int fvm_batch_create(fvm_batch **out, const fvm_ext *ext);
